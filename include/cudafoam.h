@@ -119,7 +119,13 @@ typedef struct
                                   own CTA run each inner solve inside one
                                   thread-block cluster of up to 16 CTAs,
                                   the work vectors in distributed shared
-                                  memory; 0 (default) = 16384, < 0 = never */
+                                  memory; 0 (default) = 16384, < 0 = never.
+                                  With >= 0, cudaPCG meshes from 128 cells
+                                  per SM up to what the SMs hold (about
+                                  900,000 cells, at most 6 neighbours each)
+                                  run each inner solve as one cooperative
+                                  launch with the mesh split over the SMs;
+                                  < 0 keeps the graph loop for them too    */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric
                                   V-cycle over aggregation levels (Galerkin

@@ -12,6 +12,7 @@
 #include "cf_host.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -87,6 +88,7 @@ void free_topology(cf_context* c)
     c->clones.clear();
     cf_multi_release(c);
     amg_release(c);
+    resident_release(c);
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
     c->graphs.clear();
     for (void* p : c->topoAllocs) cudaFree(p);
@@ -147,10 +149,19 @@ void rcm_order(int32_t n, const int32_t* low, const int32_t* upp, const int32_t*
                const int32_t* los, const int32_t* losS, std::vector<int32_t>& perm)
 {
     std::vector<int32_t> deg(n);
-    for (int32_t i = 0; i < n; ++i) deg[i] = (own[i + 1] - own[i]) + (losS[i + 1] - losS[i]);
+    // neighbours of every cell side by side (owner side, then neighbour
+    // side): the passes below walk the graph up to seven times
+    std::vector<int32_t> start((size_t)n + 1, 0), adj(2 * (size_t)own[n]);
+    for (int32_t i = 0; i < n; ++i)
+    {
+        int32_t at = start[i];
+        for (int32_t f = own[i]; f < own[i + 1]; ++f) adj[at++] = upp[f];
+        for (int32_t k = losS[i]; k < losS[i + 1]; ++k) adj[at++] = low[los[k]];
+        start[i + 1] = at;
+        deg[i] = at - start[i];
+    }
     auto for_nbrs = [&](int32_t v, auto&& fn) {
-        for (int32_t f = own[v]; f < own[v + 1]; ++f) fn(upp[f]);
-        for (int32_t k = losS[v]; k < losS[v + 1]; ++k) fn(low[los[k]]);
+        for (int32_t q = start[v]; q < start[v + 1]; ++q) fn(adj[q]);
     };
     std::vector<int32_t> mark(n, -1);  // search stamp
     std::vector<char> done(n, 0);
@@ -292,34 +303,35 @@ int build_layout(int32_t n, int32_t nf, const int32_t* low, const int32_t* upp,
     }
     L.col.assign((size_t)std::max(nnzp, 1LL), -1);
     L.eface.assign((size_t)std::max(nnzp, 1LL), -1);
-    int32_t maxw = 0;
-    for (int32_t r = 0; r < n; ++r)
-    {
-        const int32_t i = perm[r];
-        const int32_t s = r / SLICE;
-        const int32_t lane = r % SLICE;
-        int32_t k = 0;
-        for (int32_t f = own[i]; f < own[i + 1]; ++f, ++k)
+    const int32_t maxw = wmax;
+    host_chunks(n, host_threads(n), [&](int r0, int r1) {
+        for (int32_t r = r0; r < r1; ++r)
         {
-            const size_t e = (size_t)L.sliceOff[s] + (size_t)SLICE * k + lane;
-            L.col[e] = iperm[upp[f]];
-            L.eface[e] = f;
+            const int32_t i = perm[r];
+            const int32_t s = r / SLICE;
+            const int32_t lane = r % SLICE;
+            int32_t k = 0;
+            for (int32_t f = own[i]; f < own[i + 1]; ++f, ++k)
+            {
+                const size_t e = (size_t)L.sliceOff[s] + (size_t)SLICE * k + lane;
+                L.col[e] = iperm[upp[f]];
+                L.eface[e] = f;
+            }
+            for (int32_t q = losS[i]; q < losS[i + 1]; ++q, ++k)
+            {
+                const int32_t f = los[q];
+                const size_t e = (size_t)L.sliceOff[s] + (size_t)SLICE * k + lane;
+                L.col[e] = (int32_t)((uint32_t)iperm[low[f]] | 0x80000000u);
+                L.eface[e] = f;
+            }
+            for (int32_t x = 0; x < nExtra(i); ++x, ++k)
+            {
+                const size_t e = (size_t)L.sliceOff[s] + (size_t)SLICE * k + lane;
+                L.col[e] = xCol[xStart[i] + x];
+                L.eface[e] = xFace[xStart[i] + x];
+            }
         }
-        for (int32_t q = losS[i]; q < losS[i + 1]; ++q, ++k)
-        {
-            const int32_t f = los[q];
-            const size_t e = (size_t)L.sliceOff[s] + (size_t)SLICE * k + lane;
-            L.col[e] = (int32_t)((uint32_t)iperm[low[f]] | 0x80000000u);
-            L.eface[e] = f;
-        }
-        for (int32_t x = 0; x < nExtra(i); ++x, ++k)
-        {
-            const size_t e = (size_t)L.sliceOff[s] + (size_t)SLICE * k + lane;
-            L.col[e] = xCol[xStart[i] + x];
-            L.eface[e] = xFace[xStart[i] + x];
-        }
-        maxw = std::max(maxw, k);
-    }
+    });
     L.nslices = nslices;
     L.nnzp = nnzp;
     L.maxw = maxw;
@@ -655,77 +667,64 @@ extern "C" int cf_set_topology(cf_context* c, int32_t n, int32_t nf, const int32
     // synchronisation below)
     std::vector<short> col16((size_t)std::max(nnzp, 1LL), COL16_PAD);
     std::vector<short> pcol16;
-    {
-        bool fits = true;
-        for (int32_t sl = 0; sl < nslices && fits; ++sl)
-        {
-            const int32_t b0 = sliceOff[sl];
-            const int32_t w = (sliceOff[sl + 1] - b0) / SLICE;
-            for (int32_t k = 0; k < w && fits; ++k)
-                for (int32_t l = 0; l < SLICE; ++l)
-                {
-                    const int32_t e = b0 + SLICE * k + l;
-                    if (col[e] == -1) continue;
-                    const long long off = (long long)(col[e] & 0x7fffffff) - (long long)(sl * SLICE + l);
-                    if (off < -32767 || off > 32767)
-                    {
-                        fits = false;
-                        break;
-                    }
-                    col16[e] = (short)off;
-                }
-        }
-        if (fits)
-        {
-            CF_TRY(dalloc(c, &c->d_col16, col16.size()));
-            CF_CUDA(cudaMemcpyAsync(c->d_col16, col16.data(), sizeof(short) * col16.size(),
-                                    cudaMemcpyHostToDevice, c->stream));
-            // the same stream in the paired order, with a paired copy of the
-            // FP32 values (staged with them), when every slice has one width
-            // with paired kernels
-            if (L.uniformW >= PAIR_MIN_W && L.uniformW <= PAIR_MAX_W)
-            {
-                const int W = L.uniformW;
-                const long long sw = (long long)SLICE * W;
-                pcol16.assign(col16.size(), COL16_PAD);
-                for (long long e = 0; e < nnzp; ++e)
-                {
-                    const long long sl = e / sw;
-                    const int rem = (int)(e - sl * sw);
-                    pcol16[pair_index(sl * sw, W, rem / SLICE, rem % SLICE)] = col16[e];
-                }
-                CF_TRY(dalloc(c, &c->d_pcol16, pcol16.size()));
-                CF_TRY(dalloc(c, &c->d_pval32, pcol16.size()));
-                CF_CUDA(cudaMemcpyAsync(c->d_pcol16, pcol16.data(),
-                                        sizeof(short) * pcol16.size(), cudaMemcpyHostToDevice,
-                                        c->stream));
-            }
-        }
-    }
+    // (the paired copy: only where every slice has one width with paired kernels)
+    const int pw = L.uniformW >= PAIR_MIN_W && L.uniformW <= PAIR_MAX_W ? L.uniformW : 0;
+    if (pw) pcol16.assign(col16.size(), COL16_PAD);
     // locality of the cluster PCG's row split (cf_cluster.cu): the share of
     // entries whose column belongs to another CTA
-    {
-        c->clusterShift = cluster_shift(n);
-        long long entries = 0, remote = 0;
-        for (int32_t sl = 0; sl < nslices; ++sl)
+    c->clusterShift = cluster_shift(n);
+    std::atomic<bool> fits{true};
+    std::atomic<long long> entries{0}, remote{0};
+    host_chunks(nslices, host_threads(n), [&](int s0, int s1) {
+        long long ne = 0, nr = 0;
+        bool ok = true;
+        for (int32_t sl = s0; sl < s1; ++sl)
         {
             const int32_t b0 = sliceOff[sl];
             const int32_t w = (sliceOff[sl + 1] - b0) / SLICE;
             for (int32_t k = 0; k < w; ++k)
                 for (int32_t l = 0; l < SLICE; ++l)
                 {
-                    const int32_t cc = col[(size_t)b0 + SLICE * k + l];
-                    if (cc == -1) continue;
-                    ++entries;
+                    const int32_t e = b0 + SLICE * k + l;
+                    if (col[e] == -1) continue;
+                    const int32_t cc = col[e] & 0x7fffffff;
                     const int32_t row = sl * SLICE + l;
-                    if (((cc & 0x7fffffff) >> c->clusterShift) != (row >> c->clusterShift)) ++remote;
+                    ++ne;
+                    if ((cc >> c->clusterShift) != (row >> c->clusterShift)) ++nr;
+                    const int32_t off = cc - row;
+                    if (off < -32767 || off > 32767)
+                    {
+                        ok = false;
+                        continue;
+                    }
+                    col16[e] = (short)off;
+                    if (pw) pcol16[pair_index(b0, pw, k, l)] = (short)off;
                 }
         }
-        c->clusterRemote = entries ? (double)remote / (double)entries : 0.0;
+        entries += ne;
+        remote += nr;
+        if (!ok) fits = false;
+    });
+    c->clusterRemote = entries ? (double)remote / (double)entries : 0.0;
+    if (fits)
+    {
+        CF_TRY(dalloc(c, &c->d_col16, col16.size()));
+        CF_CUDA(cudaMemcpyAsync(c->d_col16, col16.data(), sizeof(short) * col16.size(),
+                                cudaMemcpyHostToDevice, c->stream));
+        // the same stream in the paired order, with a paired copy of the
+        // FP32 values (staged with them)
+        if (pw)
+        {
+            CF_TRY(dalloc(c, &c->d_pcol16, pcol16.size()));
+            CF_TRY(dalloc(c, &c->d_pval32, pcol16.size()));
+            CF_CUDA(cudaMemcpyAsync(c->d_pcol16, pcol16.data(), sizeof(short) * pcol16.size(),
+                                    cudaMemcpyHostToDevice, c->stream));
+        }
     }
     CF_CUDA(cudaMemsetAsync(c->d_D, 0, sizeof(float) * 3 * N, c->stream));
     CF_CUDA(cudaMemsetAsync(c->d_r64, 0, sizeof(double) * N, c->stream));
     CF_CUDA(cudaStreamSynchronize(c->stream));
+    CF_TRY(resident_build(c, L));
     c->hasTopo = true;
     c->lastLow = low;
     c->lastUpp = upp;

@@ -4,8 +4,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <map>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -115,6 +117,7 @@ struct cf_context
     int maxCtasPerSM = 32;
     bool coopLaunch = false;               // device supports cooperative launches
     void* amg = nullptr;                   // GAMG hierarchy of the topology (cf_amg.cu)
+    void* resident = nullptr;              // split of the mesh for resident inner solves (cf_resident.cu)
     bool amgActive = false;                // inner PCG iterations use the V-cycle
     int clusterShift = 10;                 // log2(rows per CTA) of the cluster PCG for this mesh
     double clusterRemote = 1.0;            // fraction of entries whose column lies in another CTA
@@ -163,6 +166,37 @@ struct HostLayout
     int32_t maxw = 0;
     int32_t uniformW = 0;           // every slice this wide (0: widths differ)
 };
+
+// fn(begin, end) over [0, n) in chunks on up to `threads` host threads (a
+// thread that cannot be started leaves its chunk to the calling one).  fn
+// must not throw.
+template <class F>
+void host_chunks(int n, int threads, F fn)
+{
+    std::vector<std::thread> pool;
+    const int step = std::max(1, (n + threads - 1) / threads);
+    int at = step;
+    for (; at < n; at += step)
+    {
+        try
+        {
+            pool.emplace_back(fn, at, std::min(n, at + step));
+        }
+        catch (...)
+        {
+            break;
+        }
+    }
+    fn(0, std::min(n, step));
+    for (; at < n; at += step) fn(at, std::min(n, at + step));
+    for (auto& t : pool) t.join();
+}
+
+// host threads worth starting for n rows of set-up work
+inline int host_threads(int n)
+{
+    return n < 20000 ? 1 : (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+}
 
 int check_addressing(int32_t n, int32_t nf, const int32_t* low, const int32_t* upp,
                      const int32_t* own, const int32_t* los, const int32_t* losS);
@@ -217,6 +251,18 @@ int cluster_inner(cf_context* c, int order, int maxCells, bool* ran);
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);
 int persistent_status(cf_context* c);
+
+// Inner PCG as one launch with the mesh split over the SMs (cf_resident.cu).
+// Meshes of at least RESIDENT_MIN_ROWS_PER_SM rows per SM get a split with
+// their topology; resident_inner runs and completes one inner solve (state
+// in h_st and d_st, the returned correction in d_D) when the context has
+// one and no other resident launch of the process runs on the device; *ran
+// tells whether it did.
+constexpr int RESIDENT_MIN_ROWS_PER_SM = 128;
+int resident_build(cf_context* c, const HostLayout& L);
+void resident_release(cf_context* c);
+int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,
+                   int order, int stagLimit, bool* ran);
 
 // Aggregation multigrid preconditioner of the inner PCG (cf_amg.cu):
 // hierarchy of the topology down to at most coarsestCap (<= 128) cells,

@@ -88,6 +88,8 @@ struct InnerState
     int converged, singular, stagnated, done, early;
     int sel;                        // buffer holding the returned correction
     unsigned int ticket;
+    int waitErr;                    // a bounded wait of a resident solve gave up (last field:
+                                    // set by any CTA, the others are written back without it)
 };
 
 // FP64 driver quantities (metalFoamSolver.C:101-415).

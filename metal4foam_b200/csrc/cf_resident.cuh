@@ -1,0 +1,50 @@
+// cf_resident.cuh -- the mesh split behind the resident inner PCG
+// (cf_resident.cu): host-side partition of one matrix into parts, one per
+// CTA, and the device layout the kernel reads.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <vector>
+
+#include "cf_internal.cuh"
+
+namespace cf {
+
+struct HostLayout;
+
+// One part = the rows of one CTA.  Local rows 0 .. nb-1 have a neighbour in
+// another part (their values are published), nb .. nloc-1 do not.  Local
+// indices of a gathered vector: own rows, then (from nlocP, nloc rounded up
+// to whole slices) the nh halo values, then one slot that holds 0 and that
+// padding entries name.
+struct ResPart
+{
+    int nloc, nlocP, nb, nh;
+    int rowBase;      // first padded row of the part in the part-ordered arrays
+    int haloBase;     // first halo entry in haloSlot
+    int llBase;       // slot of local row 0 in the exchange buffer
+    int pad_;
+};
+
+struct ResHost
+{
+    int W = 0;                        // entries per row (padded)
+    int slots = 0;                    // exchange slots (boundary rows of all parts)
+    int rowsP = 0;                    // padded rows of all parts
+    int maxLocP = 0, maxHalo = 0;
+    std::vector<ResPart> parts;
+    std::vector<int32_t> rowMap;      // [rowsP] internal row, -1 padding
+    std::vector<uint16_t> idx;        // [rowsP * W] local column, paired order per slice
+    std::vector<int32_t> emap;        // [rowsP * W] entry of the SELL arrays, -1 padding
+    std::vector<int32_t> haloSlot;    // exchange slot of every halo value
+};
+
+// Splits the rows of L (its internal order; `ordered`: reverse
+// Cuthill-McKee) into nparts parts of equal size (within one row).  Returns
+// false when a part would need more than 65,535 local indices or the rows
+// are wider than 8.
+bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R);
+
+}  // namespace cf

@@ -225,6 +225,33 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     {
         if (order > CF_MAX_CHEB) return fail(CF_ERR_INVALID_ARG, "chebyshevOrder too large");
     }
+    auto finish = [&]() {
+        const InnerState& st = *c->h_st;
+        float ms = 0.0f;
+        cudaEventElapsedTime(&ms, c->ev0, c->ev1);
+        if (stats)
+        {
+            stats->nIterations = st.it;
+            stats->converged = st.converged;
+            stats->singular = st.singular;
+            stats->stagnated = st.stagnated;
+            stats->finalResSum = st.finalResSum;
+            stats->tGpuSeconds = ms * 1e-3;
+            stats->tWallSeconds = wall_now() - tw0;
+        }
+        c->lastInnerKind = kind;
+        return CF_OK;
+    };
+    // the whole inner solve as one launch on the mesh's split over the SMs
+    if (kind == 0 && useGraph && clusterMax >= 0 && persistMax <= 0 && spmv_default(c) &&
+        !c->amgActive)
+    {
+        bool resident = false;
+        CF_CUDA(cudaEventRecord(c->ev0, s));
+        CF_TRY(resident_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
+        c->pendingBodyKernels = 0;
+        if (resident) return finish();
+    }
     k_inner_setup<<<1, 32, 0, s>>>(c->d_st, target, maxIter, ips, stagLimit);
     CF_LAUNCH();
     const PcgBufs B = pcg_bufs(c);
@@ -301,20 +328,7 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     if (persistent) CF_TRY(persistent_status(c));
     const InnerState& st = *c->h_st;
     if (c->pendingBodyKernels) c->launches += (long long)c->pendingBodyKernels * std::max(st.it, 1);
-    float ms = 0.0f;
-    cudaEventElapsedTime(&ms, c->ev0, c->ev1);
-    if (stats)
-    {
-        stats->nIterations = st.it;
-        stats->converged = st.converged;
-        stats->singular = st.singular;
-        stats->stagnated = st.stagnated;
-        stats->finalResSum = st.finalResSum;
-        stats->tGpuSeconds = ms * 1e-3;
-        stats->tWallSeconds = wall_now() - tw0;
-    }
-    c->lastInnerKind = kind;
-    return CF_OK;
+    return finish();
 }
 
 int check_ready(cf_context* c)

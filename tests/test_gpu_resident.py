@@ -1,0 +1,180 @@
+"""Resident inner PCG (meshes of 128 cells per SM up to what the SMs hold):
+the mesh split over the SMs, one cooperative launch per inner solve.  Every
+row is formed with the graph loop's operations in the graph loop's order and
+the scalars are rounded to FP32 before they are used, so the correction is
+the graph loop's (clusterMaxCells < 0) bit for bit although the FP64 sums fold
+in another order.  The sizes sit at the edges: the smallest mesh that is
+split, the first that needs another row per thread, the ones that leave
+registers for shared memory, and the first too large."""
+import threading
+
+import numpy as np
+import pytest
+
+from metal4foam_b200 import _lib, mesh
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("initialResidual", "finalResidual", "nIterations", "nRestarts", "converged", "singular",
+          "stagnated", "deflated", "polished", "normFactor", "residualL2", "chebBeta")
+
+
+def sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def context(s):
+    ctx = _lib.Context(0)
+    ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
+    ctx.set_coeffs(s.diag, s.upper, None)
+    return ctx
+
+
+def solve(ctx, s, cluster=0, **kw):
+    x = s.psi.copy()
+    l0 = ctx.kernel_launches()
+    p = ctx.solve(_lib.CF_SOLVER_PCG, x, s.source,
+                  _lib.default_options(clusterMaxCells=cluster, **kw))
+    return x, p, ctx.kernel_launches() - l0
+
+
+def chain_of_grids(cells, seed):
+    """Two unconnected grids, one of them 2 x 3 cells across."""
+    a = mesh.structured_faces((2, 3, cells // 12))
+    b = mesh.structured_faces((30, cells // 60))
+    na, nb = 6 * (cells // 12), 30 * (cells // 60)
+    low = np.concatenate([a[0], b[0] + na])
+    upp = np.concatenate([a[1], b[1] + na])
+    n = na + nb
+    rng = np.random.default_rng(seed)
+    addr = mesh.ldu_addressing(n, low, upp)
+    upper = -rng.uniform(0.5, 2.0, addr.nf)
+    diag = 0.01 - (np.bincount(low, upper, n) + np.bincount(upp, upper, n))
+    return mesh.LduSystem("chain", addr, diag, upper, None, rng.standard_normal(n), np.zeros(n))
+
+
+def random_graph(n, seed):
+    """At most six random neighbours per cell: no locality to find."""
+    rng = np.random.default_rng(seed)
+    pairs = np.concatenate([np.stack([np.arange(n), rng.permutation(n)], 1) for _ in range(3)])
+    pairs = pairs[pairs[:, 0] != pairs[:, 1]]
+    key = np.unique(np.minimum(pairs[:, 0], pairs[:, 1]) * n + np.maximum(pairs[:, 0], pairs[:, 1]))
+    low, upp = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    addr = mesh.ldu_addressing(n, low, upp)
+    upper = -rng.uniform(0.5, 2.0, addr.nf)
+    diag = 0.05 - (np.bincount(low, upper, n) + np.bincount(upp, upper, n))
+    return mesh.LduSystem("random", addr, diag, upper, None, rng.standard_normal(n), np.zeros(n))
+
+
+CASES = {
+    "first_size": (lambda m: mesh.poisson2d(128, m, seed=1), {}),
+    "one_row_each": (lambda m: mesh.varcoeff3d((16, 16, m), seed=2, permute=True), {}),
+    "two_rows": (lambda m: mesh.varcoeff3d((16, 16, m + 1), seed=3), dict(deflate="off")),
+    "prism_rcm": (lambda m: mesh.prism3d((41, 37, 29), seed=4), dict(tolerance=1e-9)),
+    "jacobi": (lambda m: mesh.poisson2d(211, 307, seed=5),
+               dict(chebyshevOrder=1, maxIter=3000)),
+    "order2_ips3": (lambda m: mesh.varcoeff3d((37, 35, 33), seed=6, permute=True),
+                    dict(chebyshevOrder=2, iterationsPerSync=3)),
+    "max_iter": (lambda m: mesh.varcoeff3d((41, 40, 39), seed=7, permute=True),
+                 dict(maxIter=17, maxRestarts=2)),
+    "unconnected": (lambda m: chain_of_grids(150 * m, 8), {}),
+    "random_graph": (lambda m: random_graph(140 * m, 9), {}),
+    "rows_10": (lambda m: mesh.poisson2d(16 * m, 160, seed=10), dict(chebyshevOrder=4)),
+    "shared_rows": (lambda m: mesh.varcoeff3d((16 * m // 10, 20, 81), seed=11), {}),
+    "last_size": (lambda m: mesh.varcoeff3d((m, 64, 88), seed=12), dict(maxIter=60)),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_resident_equals_graph(require_gpu, name):
+    make, kw = CASES[name]
+    s = make(sms())
+    ctx = context(s)
+    xg, pg, lg = solve(ctx, s, -1, **kw)
+    xr, pr, lr = solve(ctx, s, **kw)
+    assert lr < lg and lr <= 10 * (pr.nRestarts + 2), (lr, lg)     # one launch per inner solve
+    for f in FIELDS:
+        assert getattr(pr, f) == getattr(pg, f), (f, getattr(pr, f), getattr(pg, f))
+    assert np.array_equal(xr, xg)
+    # (another 1e-12: the FP64 sum of n FP32 magnitudes in another order)
+    assert pr.finalResSum32 == pytest.approx(pg.finalResSum32, rel=1e-12)
+    ctx.close()
+
+
+def test_resident_size_limits(require_gpu):
+    """Just below the first size and just above the last: the graph loop
+    (same launches with and without)."""
+    m = sms()
+    for s in (mesh.varcoeff3d((128, m - 1), seed=1, permute=False),
+              mesh.varcoeff3d((m, 64, 97), seed=2, permute=False)):
+        ctx = context(s)
+        _, pg, lg = solve(ctx, s, -1, maxIter=40)
+        _, pr, lr = solve(ctx, s, maxIter=40)
+        assert lr == lg and pr.nIterations == pg.nIterations
+        ctx.close()
+
+
+def test_resident_inner_entry_new_coeffs_and_transpose(require_gpu):
+    """cf_pcg runs through it too; new coefficients, a staged transpose and a
+    new topology on the same context are picked up."""
+    s = mesh.varcoeff3d((40, 30, 20), seed=13, permute=True)
+    ctx = context(s)
+    st = ctx.pcg(s.source, 1e-3 * np.abs(s.source).sum(), 200, chebOrder=8, chebBeta=2.0)
+    d0 = ctx.delta(s.n)
+    assert st.converged
+    ctx.set_spmv_config(blockSize=128)            # the graph loop in another launch shape
+    st1 = ctx.pcg(s.source, 1e-3 * np.abs(s.source).sum(), 200, chebOrder=8, chebBeta=2.0)
+    assert abs(st1.nIterations - st.nIterations) <= 1
+    assert np.linalg.norm(ctx.delta(s.n) - d0) <= 1e-3 * np.linalg.norm(d0)
+    ctx.set_spmv_config()
+    s2 = mesh.varcoeff3d((40, 30, 20), seed=14, permute=True)
+    ctx.set_topology(s2.addr.n, s2.addr.nf, *s2.addr.arrays())
+    for scale in (1.0, 3.0):
+        ctx.set_coeffs(scale * s2.diag, scale * s2.upper, None)
+        for on in (False, True):
+            ctx.set_transpose(on)
+            xg, pg, _ = solve(ctx, s2, -1)
+            xr, pr, _ = solve(ctx, s2)
+            assert np.array_equal(xr, xg) and pr.nIterations == pg.nIterations
+        ctx.set_transpose(False)
+    ctx.close()
+
+
+def test_resident_wait_runs_out(require_gpu):
+    """With a wait limit of one poll a CTA gives up on its neighbours: the
+    launch ends and the inner solve runs through the graph loop instead."""
+    s = mesh.varcoeff3d((40, 40, 40), seed=15, permute=True)
+    ctx = context(s)
+    xg, pg, lg = solve(ctx, s, -1)
+    ctx.set_wait_limit(1)
+    x1, p1, l1 = solve(ctx, s)
+    assert l1 > lg and np.array_equal(x1, xg) and p1.nIterations == pg.nIterations
+    ctx.set_wait_limit(0)
+    xr, pr, lr = solve(ctx, s)
+    assert lr < lg and np.array_equal(xr, xg) and pr.nIterations == pg.nIterations
+    ctx.close()
+
+
+def test_resident_from_two_threads(require_gpu):
+    """One resident launch at a time per device: solves on other threads take
+    the graph loop meanwhile, with the same result."""
+    ss = [mesh.varcoeff3d((40, 40, 20 + k), seed=20 + k, permute=True) for k in range(3)]
+    ctxs = [context(s) for s in ss]
+    ref = [solve(c, s, -1) for c, s in zip(ctxs, ss)]
+    out = [[] for _ in ss]
+
+    def work(k):
+        for _ in range(5):
+            out[k].append(solve(ctxs[k], ss[k]))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(ss))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(len(ss)):
+        assert len(out[k]) == 5
+        for x, p, _ in out[k]:
+            assert np.array_equal(x, ref[k][0]) and p.nIterations == ref[k][1].nIterations
+        ctxs[k].close()
