@@ -113,19 +113,17 @@ typedef struct
                                   are at most this many, the inner loop of
                                   every system runs as one cooperative
                                   launch per restart; 0 (default): never   */
-    int32_t clusterMaxCells;   /* cudaPCG with graph = 1: meshes up to this
-                                  many cells (at most 16384, one row per
-                                  thread) whose columns lie mostly in their
-                                  own CTA run each inner solve inside one
-                                  thread-block cluster of up to 16 CTAs,
-                                  the work vectors in distributed shared
-                                  memory; 0 (default) = 16384, < 0 = never.
-                                  With >= 0, cudaPCG meshes from 128 cells
-                                  per SM up to what the SMs hold (about
-                                  900,000 cells, at most 6 neighbours each)
-                                  run each inner solve as one cooperative
-                                  launch with the mesh split over the SMs;
-                                  < 0 keeps the graph loop for them too    */
+    int32_t clusterMaxCells;   /* cudaPCG with graph = 1.  0 (default): meshes
+                                  of at most 16384 cells whose columns lie
+                                  mostly in their own CTA run each inner
+                                  solve inside one thread-block cluster of
+                                  up to 16 CTAs; meshes with at most 6
+                                  neighbours per cell, from 128 cells per SM
+                                  on, too while they fit one cluster, and up
+                                  to what the SMs hold (about 900,000 cells)
+                                  as one cooperative launch with the mesh
+                                  split over the SMs.  < 0: the graph loop
+                                  always                                   */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric
                                   V-cycle over aggregation levels (Galerkin

@@ -1,5 +1,6 @@
 // cf_cluster.cu -- the inner PCG of a small mesh inside ONE thread-block
-// cluster.
+// cluster, for meshes with more than six neighbours per cell (the others:
+// cf_clupcg.cu).
 //
 // A mesh of up to 16,384 cells fits one cluster of up to 16 CTAs x 1024
 // threads, one row per thread: CTA k owns the rows [k RPC, (k + 1) RPC) (RPC

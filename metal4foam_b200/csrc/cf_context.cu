@@ -89,6 +89,7 @@ void free_topology(cf_context* c)
     cf_multi_release(c);
     amg_release(c);
     resident_release(c);
+    clu_release(c);
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
     c->graphs.clear();
     for (void* p : c->topoAllocs) cudaFree(p);
@@ -725,6 +726,11 @@ extern "C" int cf_set_topology(cf_context* c, int32_t n, int32_t nf, const int32
     CF_CUDA(cudaMemsetAsync(c->d_r64, 0, sizeof(double) * N, c->stream));
     CF_CUDA(cudaStreamSynchronize(c->stream));
     CF_TRY(resident_build(c, L));
+    if (n <= CLU_MAX_ROWS && maxw <= 6)
+    {
+        c->hostCol.swap(col);
+        c->hostSliceOff.swap(sliceOff);
+    }
     c->hasTopo = true;
     c->lastLow = low;
     c->lastUpp = upp;

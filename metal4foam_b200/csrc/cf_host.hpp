@@ -118,6 +118,10 @@ struct cf_context
     bool coopLaunch = false;               // device supports cooperative launches
     void* amg = nullptr;                   // GAMG hierarchy of the topology (cf_amg.cu)
     void* resident = nullptr;              // split of the mesh for resident inner solves (cf_resident.cu)
+    void* clu = nullptr;                   // split of a small mesh over one cluster (cf_clupcg.cu)
+    bool cluTried = false;                 // the split has been made, or cannot be
+    std::vector<int32_t> hostCol;          // host copy of the columns, kept for that split
+    std::vector<int32_t> hostSliceOff;
     bool amgActive = false;                // inner PCG iterations use the V-cycle
     int clusterShift = 10;                 // log2(rows per CTA) of the cluster PCG for this mesh
     double clusterRemote = 1.0;            // fraction of entries whose column lies in another CTA
@@ -247,6 +251,13 @@ int persistent_inner(cf_context* c, int kind, int order, int maxCells, bool* ran
 // at most min(maxCells, 16384) cells whose columns lie mostly in their own
 // CTA; *ran tells whether it was launched.
 int cluster_inner(cf_context* c, int order, int maxCells, bool* ran);
+// The same for meshes with at most six neighbours per cell and up to
+// CLU_MAX_ROWS cells, matrix and vectors in registers (cf_clupcg.cu); runs
+// and completes the inner solve as resident_inner does.
+constexpr int CLU_MAX_ROWS = 40960;
+int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int ips, int order,
+              int stagLimit, bool* ran);
+void clu_release(cf_context* c);
 // log2(rows per CTA) of the cluster PCG for an n-row mesh: the smallest
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);

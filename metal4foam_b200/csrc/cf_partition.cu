@@ -189,10 +189,10 @@ void bisect(std::vector<Item>& it, int lo, int hi, int p0, int np, std::vector<i
 
 }  // namespace
 
-bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R)
+bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R, int width)
 {
-    if (L.maxw < 1 || L.maxw > 8 || nparts < 1 || nparts > n) return false;
-    const int W = L.maxw;
+    const int W = std::max(width, (int)L.maxw);
+    if (W < 1 || W > 8 || nparts < 1 || nparts > n) return false;
     const int nt = host_threads(n);
     Csr g;
     csr_of_layout(n, L, nt, g);

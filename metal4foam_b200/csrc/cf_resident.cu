@@ -25,9 +25,9 @@
 //    shared memory (512 threads of up to 12 rows).
 //
 // Measured on one box, us per inner iteration, graph loop / this kernel
-// (Chebyshev 8): 24K cells 3-D 28.7 / 15.7, 200K prisms 43.5 / 17.3, 262K
-// 3-D 45.0 / 18.5, 307K 2-D 43.9 / 17.7, 448K 3-D 56.0 / 29.6, 885K 3-D
-// 86.8 / 59.3; Jacobi, 262K: 17.5 / 8.3.  What is left at 24K-300K cells is
+// (Chebyshev 8): 24K cells 3-D 28.7 / 15.7, 200K prisms 43.7 / 18.0, 262K
+// 3-D 45.7 / 17.4, 307K 2-D 44.2 / 15.0, 448K 3-D 56.0 / 29.6; Jacobi, 262K:
+// 17.5 / 8.4.  What is left at 24K-300K cells is
 // the trip of a word from SM to SM through L2, 1,750 cycles there and back in
 // the median pair (measured with two CTAs bouncing one word), ten times per
 // iteration.  128^3 does not fit on the SMs: with the rest of the matrix
@@ -49,7 +49,8 @@
 // reduction, after which the caller runs the graph path instead.
 #include "cudafoam.h"
 #include "cf_host.hpp"
-#include "cf_resident.cuh"
+#include "cf_inner.cuh"
+#include "cf_cluster_ll.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -71,10 +72,7 @@ namespace cf {
 
 namespace {
 
-typedef unsigned long long u64;
-
 constexpr int RES_MAX_PARTS = 256;   // CTAs of one system at most
-constexpr int RES_GROUP = 4;         // rows whose gathers are in flight together
 constexpr int RES_MAX_ROWS = 6144;   // rows of a part at most (the last entry of CHIP)
 constexpr int RES_COPIES = 8;        // copies of every reduction word
 constexpr size_t RES_RED_WORDS = (size_t)RES_COPIES * RES_MAX_PARTS * 4;
@@ -294,113 +292,33 @@ __device__ __forceinline__ double red_total(const ResArgs& a, const ResShared& s
     return t;
 }
 
-// After the gather of {sum|r| of the last update, z.r}: the bookkeeping of
-// k_pcg_update (for iteration > 0) and of the last Chebyshev step, by one
-// thread; the others go on (they form beta themselves) and learn of the end
-// of the solve at the next reduction.
-__device__ __forceinline__ void state_after_apply(ResShared& sh, bool first, double res,
-                                                  double wArA)
-{
-    InnerState& S = sh.S;
-    if (!first)
-    {
-        S.res = res;
-        S.cur = S.nxt;
-        S.it = S.it + 1;
-        inner_sync_point(&S, true);
-    }
-    if (!S.done)
-    {
-        S.wArAold = S.wArA;
-        S.wArA = wArA;
-    }
-    sh.stop = S.done || sh.bad;
-}
-
 __device__ __forceinline__ void state_init(const ResArgs& a, ResShared& sh)
 {
-    InnerState& S = sh.S;
-    S.stagLimit = a.stagLimit > 0 ? a.stagLimit : STAG_LIMIT;
-    S.wArA = S.wArAold = S.wApA = S.alpha = S.beta = S.res = 0.0;
-    S.rA0rA = S.rA0rAold = S.rA0AyA = S.omega = S.tAtA = S.tAsA = S.resS = 0.0;
-    S.bestRes = 1.0e300;
-    S.target = a.target;
-    S.finalResSum = 0.0;
-    S.it = 0;
-    S.maxIter = a.maxIter;
-    S.ips = a.ips < 1 ? 1 : a.ips;
-    S.lastSync = 0;
-    S.noProgress = 0;
-    S.cur = S.best = 0;
-    S.nxt = 1;
-    S.converged = S.singular = S.stagnated = S.done = S.early = 0;
-    S.sel = 0;
-    S.ticket = 0u;
-    S.waitErr = 0;
+    inner_state_init(sh.S, a.target, a.maxIter, a.ips, a.stagLimit);
     sh.stop = 0;
     sh.bad = 0;
-}
-
-// k_inner_final's choice; the state goes back without its error word
-__device__ __forceinline__ void state_final(const ResArgs& a, ResShared& sh, int rank)
-{
-    InnerState& S = sh.S;
-    if (S.bestRes < S.finalResSum)
-    {
-        S.sel = S.best;
-        S.finalResSum = S.bestRes;
-    }
-    else
-    {
-        S.sel = S.cur;
-    }
-    if (rank == 0)
-    {
-        const int err = *(volatile int*)&a.st->waitErr;
-        S.waitErr = err;
-        InnerState t = S;
-        // field by field up to waitErr: another CTA may set it at any time
-        memcpy((void*)a.st, (const void*)&t, offsetof(InnerState, waitErr));
-    }
-}
-
-template <int W>
-__device__ __forceinline__ float row_apply(const unsigned int (&ix)[(W + 1) / 2],
-                                           const float (&v)[W], const float* x, float acc)
-{
-    float t[W];
-#pragma unroll
-    for (int k = 0; k < W; ++k)
-        t[k] = x[(k & 1) ? (ix[k >> 1] >> 16) : (ix[k >> 1] & 0xffffu)];
-#pragma unroll
-    for (int k = 0; k < W; ++k) acc = __fadd_rn(acc, __fmul_rn(v[k], t[k]));
-    return acc;
-}
-
-// entries of local row l (paired order), base = (rowBase + slice start) W
-template <int W>
-__device__ __forceinline__ void row_index(const unsigned short* idx, long long sb, int lane,
-                                          unsigned int (&ix)[(W + 1) / 2])
-{
-#pragma unroll
-    for (int g = 0; g < W / 2; ++g)
-        ix[g] = *reinterpret_cast<const unsigned int*>(idx + sb + 64 * g + 2 * lane);
-    if constexpr (W & 1) ix[W / 2] = idx[sb + 32 * (W - 1) + lane];
 }
 
 // ------------------------------------------------- parts that fit on the SM
 
 // R rows per thread (row i of a thread: local row tid + i T).  The matrix
 // entries of the first RM of them stay in registers, those of the others in
-// shared memory; diag, 1/diag, r and w always stay in registers.  Rows are
-// worked in groups of RES_GROUP: a group's gathers are all issued before its
-// first result is stored (the compiler cannot tell the two z buffers apart).
+// shared memory; diag, 1/diag, r and w always stay in registers.  Results go
+// to the next z only after the gathers from the current one (the compiler
+// cannot tell the two buffers apart).
 template <int W, int R, int RM, int TB>
 __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResArgs a)
 {
     extern __shared__ float zmem[];
     __shared__ ResShared sh;
     constexpr bool LEAN = R * TB > 2560;   // z, delta and q of a row are not kept in registers
+    // Rows of the first RB thread rows are finished and published one after
+    // the other, the rest (rows no other part reads, mostly) in whatever
+    // order keeps most gathers in flight: a part's boundary is 6% of its rows
+    // on 2-D meshes and up to half on 3-D ones.  us per iteration with RB 0 /
+    // 1 / 2 / 4: 262K 3-D 19.7 / 18.6 / 17.1 / 17.4, 200K prisms 19.3 / 19.1 /
+    // 18.7 / 18.0, 307K 2-D 15.0 / 14.9 / 15.1 / 15.0.
+    constexpr int RB = W == 4 ? 1 : 4;
     const int tid = threadIdx.x;
     const int T = blockDim.x;
     const int rank = blockIdx.x;
@@ -428,6 +346,7 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
     for (int q = 0; q < RES_HQ; ++q)
         hs[q] = tid + q * T < P.nh ? a.haloSlot[P.haloBase + tid + q * T] : -1;
     for (int h = tid; h < P.nh; h += T) pb[P.nlocP + h] = 0.0f;
+    for (int l = P.nloc + tid; l < P.nlocP; l += T) zc[l] = zn[l] = pb[l] = 0.0f;
 
     constexpr int RMA = RM > 0 ? RM : 1;
     constexpr int RK = LEAN ? 1 : R;
@@ -535,30 +454,50 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
             __syncthreads();
             ++ep;
             const bool last = j == a.order - 1;
-#pragma unroll
-            for (int i0 = 0; i0 < R; i0 += RES_GROUP)
+            if constexpr (!LEAN)
             {
-                float zv[RES_GROUP];
+                // (rows past the part's end hold zeros and need no test)
 #pragma unroll
-                for (int i = i0; i < i0 + RES_GROUP && i < R; ++i)
+                for (int i = 0; i < R; ++i)
                 {
-                    const int l = tid + i * T;
-                    if (l >= P.nloc) continue;
-                    const float zl = LEAN ? zc[l] : z[LEAN ? 0 : i];
-                    const float av = row(i, l, zc, __fmul_rn(dg[i], zl));
-                    const float wn = __fadd_rn(__fmul_rn(c2, w[i]),
-                                               __fmul_rn(__fmul_rn(c3, rd[i]), __fsub_rn(r[i], av)));
-                    zv[i - i0] = __fadd_rn(zl, wn);
-                    w[i] = wn;
-                    if (!LEAN) z[LEAN ? 0 : i] = zv[i - i0];
-                    if (l < P.nb) st_word(lw + P.llBase + l, __float_as_uint(zv[i - i0]), ep);
-                    if (last) accZ += (double)zv[i - i0] * (double)r[i];
+                    const float av = row(i, tid + i * T, zc, __fmul_rn(dg[i], z[i]));
+                    w[i] = __fadd_rn(__fmul_rn(c2, w[i]),
+                                     __fmul_rn(__fmul_rn(c3, rd[i]), __fsub_rn(r[i], av)));
+                    z[i] = __fadd_rn(z[i], w[i]);
+                    if (tid + i * T < P.nb)
+                        st_word(lw + P.llBase + tid + i * T, __float_as_uint(z[i]), ep);
+                    if (i < RB) __syncwarp();
                 }
 #pragma unroll
-                for (int i = i0; i < i0 + RES_GROUP && i < R; ++i)
+                for (int i = 0; i < R; ++i)
                 {
-                    const int l = tid + i * T;
-                    if (l < P.nloc) zn[l] = zv[i - i0];
+                    if (tid + i * T < P.nloc) zn[tid + i * T] = z[i];
+                    if (last) accZ += (double)z[i] * (double)r[i];
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int i0 = 0; i0 < R; i0 += 4)
+                {
+                    float zv[4];
+#pragma unroll
+                    for (int i = i0; i < i0 + 4 && i < R; ++i)
+                    {
+                        const int l = tid + i * T;
+                        if (l >= P.nloc) continue;
+                        const float zl = zc[l];
+                        const float av = row(i, l, zc, __fmul_rn(dg[i], zl));
+                        const float wn = __fadd_rn(
+                            __fmul_rn(c2, w[i]), __fmul_rn(__fmul_rn(c3, rd[i]), __fsub_rn(r[i], av)));
+                        zv[i - i0] = __fadd_rn(zl, wn);
+                        w[i] = wn;
+                        if (l < P.nb) st_word(lw + P.llBase + l, __float_as_uint(zv[i - i0]), ep);
+                        if (last) accZ += (double)zv[i - i0] * (double)r[i];
+                    }
+#pragma unroll
+                    for (int i = i0; i < i0 + 4 && i < R; ++i)
+                        if (tid + i * T < P.nloc) zn[tid + i * T] = zv[i - i0];
                 }
             }
             swap_ptr(lw, lr);
@@ -591,34 +530,44 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
         ++ep;
         double acc[1] = {0.0};
         float q[RK];
-#pragma unroll
-        for (int i0 = 0; i0 < R; i0 += RES_GROUP)
+        if constexpr (!LEAN)
         {
-            float qv[RES_GROUP];
 #pragma unroll
-            for (int i = i0; i < i0 + RES_GROUP && i < R; ++i)
+            for (int i = 0; i < R; ++i)
             {
-                const int l = tid + i * T;
-                if (l >= P.nloc) continue;
-                const float pr = pb[l];
-                qv[i - i0] = row(i, l, pb, __fmul_rn(dg[i], pr));
-                acc[0] += (double)pr * (double)qv[i - i0];
-                if (!LEAN) q[LEAN ? 0 : i] = qv[i - i0];
+                const float pr = pb[min(tid + i * T, zs - 1)];
+                q[i] = row(i, tid + i * T, pb, __fmul_rn(dg[i], pr));
+                acc[0] += (double)pr * (double)q[i];
             }
-            if (LEAN)
-            {
+        }
+        else
+        {
 #pragma unroll
-                for (int i = i0; i < i0 + RES_GROUP && i < R; ++i)
+            for (int i0 = 0; i0 < R; i0 += 4)
+            {
+                float qv[4];
+#pragma unroll
+                for (int i = i0; i < i0 + 4 && i < R; ++i)
                 {
                     const int l = tid + i * T;
-                    if (l < P.nloc) zn[l] = qv[i - i0];
+                    if (l >= P.nloc) continue;
+                    const float pr = pb[l];
+                    qv[i - i0] = row(i, l, pb, __fmul_rn(dg[i], pr));
+                    acc[0] += (double)pr * (double)qv[i - i0];
                 }
+#pragma unroll
+                for (int i = i0; i < i0 + 4 && i < R; ++i)
+                    if (tid + i * T < P.nloc) zn[tid + i * T] = qv[i - i0];
             }
         }
         {
             red_send<1>(acc, redB, rank, ep, sh, tid, T);
             // the bookkeeping of the update before, while p.q is on its way
-            if (tid == T - 1) state_after_apply(sh, first, rsum, wArA);
+            if (tid == T - 1) 
+            {
+                inner_after_apply(sh.S, first, rsum, wArA);
+                sh.stop = sh.S.done || sh.bad;
+            }
             red_recv<1>(a, redB, rank, ep, sh, tid, T);
             __syncthreads();
             first = false;
@@ -632,17 +581,17 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
         accR = accZ = 0.0;
         float* dn = a.dw + (size_t)nxt * a.rowsP + P.rowBase;
 #pragma unroll
-        for (int i0 = 0; i0 < R; i0 += RES_GROUP)
+        for (int i0 = 0; i0 < R; i0 += 4)
         {
-            float dd[RES_GROUP];
+            float dd[4];
             if (LEAN)
             {
 #pragma unroll
-                for (int i = i0; i < i0 + RES_GROUP && i < R; ++i)
+                for (int i = i0; i < i0 + 4 && i < R; ++i)
                     dd[i - i0] = tid + i * T < P.nloc ? dcur[tid + i * T] : 0.0f;
             }
 #pragma unroll
-            for (int i = i0; i < i0 + RES_GROUP && i < R; ++i)
+            for (int i = i0; i < i0 + 4 && i < R; ++i)
             {
                 const int l = tid + i * T;
                 if (l >= P.nloc) continue;
@@ -666,7 +615,7 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
         }
         swap_ptr(lw, lr);
     }
-    if (tid == T - 1) state_final(a, sh, rank);
+    if (tid == T - 1) inner_finish(sh.S, a.st, rank == 0);
     __syncthreads();
     const int sel = sh.S.sel;
     const float* ds = a.dw + (size_t)sel * a.rowsP + P.rowBase;
@@ -727,7 +676,7 @@ const ChipKernel CHIP[] = {
     RES_CHIP(1, 1, 256),  RES_CHIP(2, 2, 256),  RES_CHIP(3, 3, 256), RES_CHIP(4, 4, 256),
     RES_CHIP(5, 5, 256),  RES_CHIP(6, 6, 256),  RES_CHIP(7, 7, 256), RES_CHIP(8, 8, 256),
     RES_CHIP(9, 9, 256),  RES_CHIP(10, 10, 256), RES_CHIP(6, 4, 512), RES_CHIP(8, 4, 512),
-    RES_CHIP(10, 4, 512), RES_CHIP(12, 4, 512)};
+    RES_CHIP(10, 5, 512), RES_CHIP(12, 5, 512)};
 
 template <class T>
 int up(cf_context* c, ResPlan* p, T** d, const T* h, size_t count)

@@ -44,7 +44,8 @@ struct ResHost
 // Splits the rows of L (its internal order; `ordered`: reverse
 // Cuthill-McKee) into nparts parts of equal size (within one row).  Returns
 // false when a part would need more than 65,535 local indices or the rows
-// are wider than 8.
-bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R);
+// are wider than 8.  Rows are padded to `width` entries at least.
+bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R,
+                   int width = 0);
 
 }  // namespace cf

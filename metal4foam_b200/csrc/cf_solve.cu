@@ -248,7 +248,13 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     {
         bool resident = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
-        CF_TRY(resident_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
+        // in one cluster up to 16,384 rows when their columns lie mostly in
+        // their own CTA (as the other cluster form) and from where the split
+        // over all SMs starts
+        if (c->n <= 16384 ? c->clusterRemote <= 0.25 : c->resident && c->n <= CLU_MAX_ROWS)
+            CF_TRY(clu_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
+        if (!resident)
+            CF_TRY(resident_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
         c->pendingBodyKernels = 0;
         if (resident) return finish();
     }

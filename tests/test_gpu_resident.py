@@ -1,6 +1,6 @@
-"""Resident inner PCG (meshes of 128 cells per SM up to what the SMs hold):
-the mesh split over the SMs, one cooperative launch per inner solve.  Every
-row is formed with the graph loop's operations in the graph loop's order and
+"""Resident inner PCG: the mesh split over the CTAs of one cluster (small
+meshes) or over the SMs (128 cells per SM up to what the SMs hold), one
+launch per inner solve.  Every row is formed with the graph loop's operations in the graph loop's order and
 the scalars are rounded to FP32 before they are used, so the correction is
 the graph loop's (clusterMaxCells < 0) bit for bit although the FP64 sums fold
 in another order.  The sizes sit at the edges: the smallest mesh that is
@@ -99,6 +99,62 @@ def test_resident_equals_graph(require_gpu, name):
     assert np.array_equal(xr, xg)
     # (another 1e-12: the FP64 sum of n FP32 magnitudes in another order)
     assert pr.finalResSum32 == pytest.approx(pg.finalResSum32, rel=1e-12)
+    ctx.close()
+
+
+def chain_1d(n, seed):
+    low = np.arange(n - 1, dtype=np.int32)
+    addr = mesh.ldu_addressing(n, low, low + 1)
+    rng = np.random.default_rng(seed)
+    upper = -rng.uniform(0.5, 2.0, n - 1)
+    diag = 0.1 - (np.bincount(low, upper, n) + np.bincount(low + 1, upper, n))
+    return mesh.LduSystem("chain", addr, diag, upper, None, rng.standard_normal(n), np.zeros(n))
+
+
+# one cluster: one CTA, its last row, a second CTA, every number of rows per
+# thread, no faces at all, the largest meshes of each width
+CLUSTER = {
+    "one_cell": (lambda: chain_1d(1, 1), {}),
+    "one_cta": (lambda: mesh.poisson2d(16, 16, seed=2), {}),
+    "two_ctas": (lambda: chain_1d(257, 3), dict(chebyshevOrder=3)),
+    "sixteen_ctas": (lambda: mesh.poisson2d(63, 65, seed=4), dict(deflate="off", tolerance=1e-7)),
+    "two_rows": (lambda: mesh.varcoeff3d((100, 71), seed=5, permute=False), {}),
+    "three_rows_3d": (lambda: mesh.varcoeff3d((25, 23, 21), seed=6, permute=False),
+                      dict(iterationsPerSync=4)),
+    "four_rows": (lambda: mesh.poisson2d(128, 128, seed=7), dict(chebyshevOrder=4)),
+    "jacobi": (lambda: mesh.poisson2d(90, 80, seed=8), dict(chebyshevOrder=1, maxIter=3000)),
+    "max_iter": (lambda: mesh.varcoeff3d((80, 50), seed=9, permute=False),
+                 dict(maxIter=23, maxRestarts=3)),
+    "no_faces": (lambda: mesh.LduSystem("diag", mesh.ldu_addressing(
+        900, np.zeros(0, np.int32), np.zeros(0, np.int32)), np.linspace(1.0, 2.0, 900),
+        np.zeros(0), None, np.linspace(-1.0, 1.0, 900), np.zeros(900)), {}),
+    "six_rows_3d": (lambda: mesh.varcoeff3d((31, 29, 27), seed=10, permute=True), {}),
+    "last_3d": (lambda: mesh.varcoeff3d((30, 35, 26), seed=11), {}),
+    "last_prism": (lambda: mesh.prism3d((32, 32, 16), seed=12), {}),
+    "ten_rows_2d": (lambda: mesh.poisson2d(256, 160, seed=13), {}),
+}
+
+
+@pytest.mark.parametrize("name", CLUSTER)
+def test_cluster_equals_graph(require_gpu, name):
+    make, kw = CLUSTER[name]
+    s = make()
+    ctx = context(s)
+    xg, pg, lg = solve(ctx, s, -1, **kw)
+    for _ in range(2):
+        xr, pr, lr = solve(ctx, s, **kw)
+        assert lr < lg and lr <= 10 * (pr.nRestarts + 2), (lr, lg)
+        for f in FIELDS:
+            assert getattr(pr, f) == getattr(pg, f), (f, getattr(pr, f), getattr(pg, f))
+        assert np.array_equal(xr, xg)
+        assert pr.finalResSum32 == pytest.approx(pg.finalResSum32, rel=1e-12)
+    # a wait limit of one poll: the graph loop takes over, nothing else changes
+    ctx.set_wait_limit(1)
+    x1, p1, _ = solve(ctx, s, **kw)
+    assert np.array_equal(x1, xg) and p1.nIterations == pg.nIterations
+    ctx.set_wait_limit(0)
+    x2, p2, l2 = solve(ctx, s, **kw)
+    assert l2 == lr and np.array_equal(x2, xg)
     ctx.close()
 
 
