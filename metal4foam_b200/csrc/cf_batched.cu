@@ -18,7 +18,9 @@
 // Per row the arithmetic is the single-system kernels' (same row functions),
 // so every system follows exactly the iteration it would follow alone.
 #include "cudafoam.h"
+#include "cf_cluster_ll.cuh"
 #include "cf_host.hpp"
+#include "cf_resident.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1037,6 +1039,27 @@ struct cf_batch
     InnerState* h_st = nullptr;
     int* h_counters = nullptr;
     std::map<int, cudaGraphExec_t> graphs;
+
+    // inner solves that run whole (cf_clupcg.cu, cf_resident.cu), when every
+    // system of the batch has a split: the small systems as clusters, those
+    // with the same kernel in one launch, the others each as a cooperative
+    // launch on its share of the SMs; all at once on streams of their own
+    struct Group
+    {
+        int W = 0, R = 0, ctas = 0, threads = 0;
+        size_t smem = 0;
+        std::vector<int> sys;
+        CluSys* d_list = nullptr;
+    };
+    bool whole = false;
+    int wholeOrder = -1;                   // chebyshevOrder of the uploaded lists
+    std::vector<CluPlan*> clu;
+    std::vector<ResPlan*> res;
+    std::vector<Group> groups;
+    std::vector<std::vector<int>> slots;   // systems of a share of the SMs, one after another
+    std::vector<cudaStream_t> streams;     // one per slot, then one per group
+    std::vector<cudaEvent_t> joins;
+    cudaEvent_t fork = nullptr;
 };
 
 #define CFB_CUDA(call)                                                          \
@@ -1319,6 +1342,255 @@ int persistent_loop(cf_batch* bt, int order, bool* ran)
     return CF_OK;
 }
 
+InnerRun whole_run(const cf_batch* bt, int i, int order)
+{
+    InnerRun r;
+    r.val32 = bt->d_val32;
+    r.diag32 = bt->d_diag32;
+    r.rD32 = bt->d_rD;
+    r.chebC = bt->d_chebC + (size_t)i * kChebStride;
+    r.r64 = bt->d_r64;
+    r.mean = &bt->d_drv[i].rmean;
+    r.useMean = &bt->d_drv[i].deflate;
+    r.D = bt->d_D;
+    r.dStride = bt->N;
+    r.st = bt->d_st + i;
+    r.fromState = 1;
+    r.order = order;
+    r.target = 0.0;
+    r.maxIter = r.ips = r.stagLimit = 0;
+    r.polls = 1LL << 24;
+    return r;
+}
+
+void whole_release(cf_batch* bt)
+{
+    bt->whole = false;
+    for (CluPlan* p : bt->clu) clu_plan_free(p);
+    for (ResPlan* p : bt->res) res_plan_free(p);
+    for (auto& g : bt->groups)
+        if (g.d_list) cudaFree(g.d_list);
+    for (cudaStream_t s : bt->streams) cudaStreamDestroy(s);
+    for (cudaEvent_t e : bt->joins) cudaEventDestroy(e);
+    if (bt->fork) cudaEventDestroy(bt->fork);
+    bt->clu.clear();
+    bt->res.clear();
+    bt->groups.clear();
+    bt->slots.clear();
+    bt->streams.clear();
+    bt->joins.clear();
+    bt->fork = nullptr;
+}
+
+// Splits for the whole inner solves of every system (bt->whole stays false
+// when a system has rows wider than six entries or is too large).  The CTAs
+// of a system: as few rows each (the kernels' steps cost less) as lets all
+// systems run side by side, one CTA per SM.
+int whole_build(cf_batch* bt, int reorder)
+{
+    if (!bt->coop || bt->S < 1) return CF_OK;
+    const int S = bt->S;
+    struct Level
+    {
+        int cluRows, resRows;
+    };
+    const Level levels[] = {{256, 768}, {512, 1280}, {1024, 1792}, {2560, 2560}};
+    std::vector<int> ctas(S);
+    std::vector<char> isClu(S);
+    for (int i = 0; i < S; ++i)
+    {
+        const auto& y = bt->sys[i];
+        if (y.L.maxw > 6) return CF_OK;
+        isClu[i] = (long long)y.n * std::max(4, (int)y.L.maxw) <= 163840;
+    }
+    int resMax = bt->numSMs;   // SMs of the cooperative launches
+    for (const Level& lv : levels)
+    {
+        long long total = 0;
+        long long resTotal = 0;
+        for (int i = 0; i < S; ++i)
+        {
+            const int n = bt->sys[i].n;
+            if (isClu[i])
+            {
+                int k = 1;
+                while (k < CLU_MAX_CTAS && n > (long long)k * lv.cluRows) k *= 2;
+                ctas[i] = k;
+            }
+            else
+            {
+                ctas[i] = std::max(8, (n + lv.resRows - 1) / lv.resRows);
+                if (ctas[i] > bt->numSMs) return CF_OK;
+                resTotal += ctas[i];
+            }
+            total += ctas[i];
+        }
+        if (total <= bt->numSMs) break;
+        // the last level: clusters wait for SMs, a quarter of them theirs
+        resMax = resTotal < total ? bt->numSMs - bt->numSMs / 4 : bt->numSMs;
+    }
+    bt->clu.assign(S, nullptr);
+    bt->res.assign(S, nullptr);
+    std::vector<int> rc(S, CF_OK);
+    std::vector<std::string> msg(S);
+    host_chunks(S, std::min(S, host_threads(1 << 20)), [&](int b, int e) {
+        cudaSetDevice(bt->device);
+        for (int i = b; i < e; ++i)
+        {
+            const auto& y = bt->sys[i];
+            const bool ordered =
+                reorder == CF_REORDER_RCM || (reorder == CF_REORDER_AUTO && y.n > 65536);
+            rc[i] = isClu[i] ? clu_plan_build(y.n, y.L, ordered, ctas[i], y.ent0, y.row0,
+                                              bt->stream, &bt->clu[i])
+                             : res_plan_build(bt->device, y.n, y.L, ordered, ctas[i], y.ent0,
+                                              y.row0, bt->stream, &bt->res[i]);
+            if (rc[i] != CF_OK) msg[i] = cf_last_error();
+        }
+    });
+    for (int i = 0; i < S; ++i)
+        if (rc[i] != CF_OK) return fail(rc[i], msg[i]);
+    for (int i = 0; i < S; ++i)
+        if (!bt->clu[i] && !bt->res[i])
+        {
+            whole_release(bt);
+            return CF_OK;
+        }
+    // shares of the SMs: the largest systems open one each, the others follow
+    // on the least loaded share that is large enough
+    std::vector<int> order(S);
+    for (int i = 0; i < S; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int a, int b) { return bt->sys[a].n > bt->sys[b].n; });
+    int used = 0;
+    std::vector<int> size;
+    std::vector<long long> load;
+    for (int i : order)
+    {
+        if (!bt->res[i]) continue;
+        if (used + ctas[i] <= resMax || size.empty())
+        {
+            used += ctas[i];
+            size.push_back(ctas[i]);
+            load.push_back(bt->sys[i].n);
+            bt->slots.push_back({i});
+            continue;
+        }
+        int best = 0;   // (the first share is the largest)
+        for (int k = 1; k < (int)size.size(); ++k)
+            if (size[k] >= ctas[i] && load[k] < load[best]) best = k;
+        bt->slots[best].push_back(i);
+        load[best] += bt->sys[i].n;
+    }
+    for (int i : order)
+    {
+        const CluPlan* p = bt->clu[i];
+        if (!p) continue;
+        cf_batch::Group* g = nullptr;
+        for (auto& q : bt->groups)
+            if (q.W == p->W && q.R == p->R && q.ctas == p->split.ctas) g = &q;
+        if (!g)
+        {
+            bt->groups.emplace_back();
+            g = &bt->groups.back();
+            g->W = p->W;
+            g->R = p->R;
+            g->ctas = p->split.ctas;
+        }
+        g->threads = std::max(g->threads, p->threads);
+        g->smem = std::max(g->smem, p->smem);
+        g->sys.push_back(i);
+    }
+    for (auto& g : bt->groups)
+        CFB_CUDA(cudaMalloc((void**)&g.d_list, sizeof(CluSys) * g.sys.size()));
+    const size_t ns = bt->slots.size() + bt->groups.size();
+    CFB_CUDA(cudaEventCreateWithFlags(&bt->fork, cudaEventDisableTiming));
+    for (size_t k = 0; k < ns; ++k)
+    {
+        cudaStream_t s = nullptr;
+        cudaEvent_t e = nullptr;
+        CFB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        bt->streams.push_back(s);
+        CFB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        bt->joins.push_back(e);
+    }
+    bt->whole = true;
+    return CF_OK;
+}
+
+// The inner solves of all active systems, each run whole.  *ran stays false
+// when another resident launch has the device or a wait gave up (the states
+// are then as kb_outer_begin left them): the batched loop runs instead.
+int whole_loop(cf_batch* bt, const cf_options* o, bool* ran)
+{
+    *ran = false;
+    cudaStream_t s = bt->stream;
+    std::unique_lock<std::mutex> turn(res_device_lock(bt->device), std::defer_lock);
+    if (!bt->slots.empty() && !turn.try_lock()) return CF_OK;
+    const int order = o->chebyshevOrder;
+    if (bt->wholeOrder != order)
+    {
+        for (auto& g : bt->groups)
+        {
+            std::vector<CluSys> list(g.sys.size());
+            for (size_t k = 0; k < list.size(); ++k)
+            {
+                const CluPlan* p = bt->clu[g.sys[k]];
+                list[k].split = p->split;
+                list[k].run = whole_run(bt, g.sys[k], order);
+                list[k].dw = p->dw;
+            }
+            CFB_CUDA(cudaMemcpyAsync(g.d_list, list.data(), sizeof(CluSys) * list.size(),
+                                     cudaMemcpyHostToDevice, s));
+            CFB_CUDA(cudaStreamSynchronize(s));
+        }
+        bt->wholeOrder = order;
+    }
+    CFB_CUDA(cudaEventRecord(bt->fork, s));
+    size_t q = 0;
+    for (const auto& slot : bt->slots)
+    {
+        cudaStream_t t = bt->streams[q];
+        CFB_CUDA(cudaStreamWaitEvent(t, bt->fork, 0));
+        for (int i : slot)
+        {
+            CFB_TRY(res_launch(bt->res[i], whole_run(bt, i, order), t));
+            bt->launches++;
+        }
+        CFB_CUDA(cudaEventRecord(bt->joins[q], t));
+        ++q;
+    }
+    for (const auto& g : bt->groups)
+    {
+        cudaStream_t t = bt->streams[q];
+        CFB_CUDA(cudaStreamWaitEvent(t, bt->fork, 0));
+        CFB_TRY(clu_launch(g.W, g.R, g.ctas, g.threads, g.smem, nullptr, g.d_list,
+                           (int)g.sys.size(), t));
+        bt->launches++;
+        CFB_CUDA(cudaEventRecord(bt->joins[q], t));
+        ++q;
+    }
+    for (cudaEvent_t e : bt->joins) CFB_CUDA(cudaStreamWaitEvent(s, e, 0));
+    CFB_CUDA(cudaMemcpyAsync(bt->h_st, bt->d_st, sizeof(InnerState) * bt->S,
+                             cudaMemcpyDeviceToHost, s));
+    CFB_CUDA(cudaStreamSynchronize(s));
+    bool gaveUp = false;
+    for (int i = 0; i < bt->S; ++i) gaveUp = gaveUp || bt->h_st[i].waitErr;
+    if (!gaveUp)
+    {
+        *ran = true;
+        return CF_OK;
+    }
+    for (const ResPlan* p : bt->res)
+        if (p) CFB_TRY(res_reset(p, s));
+    for (int i = 0; i < bt->S; ++i)
+        CFB_CUDA(cudaMemsetAsync(&bt->d_st[i].waitErr, 0, sizeof(int), s));
+    CFB_CUDA(cudaMemsetAsync(bt->d_counters, 0, 2 * sizeof(int), s));
+    kb_outer_begin<<<sgrid(bt), 128, 0, s>>>(bt->S, bt->d_st, bt->d_drv, bt->d_counters,
+                                             o->maxIter, o->iterationsPerSync, o->stagnationLimit);
+    CFB_LAUNCH();
+    return CF_OK;
+}
+
 int batch_solve(cf_batch* bt, double* const* psi, const double* const* src, bool hostPtrs,
                 const cf_options* o, cf_performance* perf)
 {
@@ -1372,33 +1644,40 @@ int batch_solve(cf_batch* bt, double* const* psi, const double* const* src, bool
         CFB_LAUNCH();
         kb_mean<1><<<tgrid(bt, (const void*)kb_mean<1>), NT, 0, s>>>(B);
         CFB_LAUNCH();
-        if (order > 1)
-            kb_pcg_init<true><<<tgrid(bt, (const void*)kb_pcg_init<true>), NT, 0, s>>>(B);
-        else
-            kb_pcg_init<false><<<tgrid(bt, (const void*)kb_pcg_init<false>), NT, 0, s>>>(B);
-        CFB_LAUNCH();
-        kb_compact<<<1, 1024, 0, s>>>(B, 1);
-        CFB_LAUNCH();
-        CFB_TRY(fetch_counters(bt));
-        if (bt->h_counters[0] > 0)
+        bool whole = false;
+        if (bt->whole && o->graph && o->persistentMaxCells <= 0 && o->clusterMaxCells >= 0 &&
+            o->maxIter > 0)
+            CFB_TRY(whole_loop(bt, o, &whole));
+        if (!whole)
         {
-            // opt-in: the whole inner loop of all systems as one launch
-            bool ran = false;
-            if (o->graph && o->persistentMaxCells > 0 && bt->N <= o->persistentMaxCells)
-                CFB_TRY(persistent_loop(bt, order, &ran));
-            if (!ran && o->graph)
+            if (order > 1)
+                kb_pcg_init<true><<<tgrid(bt, (const void*)kb_pcg_init<true>), NT, 0, s>>>(B);
+            else
+                kb_pcg_init<false><<<tgrid(bt, (const void*)kb_pcg_init<false>), NT, 0, s>>>(B);
+            CFB_LAUNCH();
+            kb_compact<<<1, 1024, 0, s>>>(B, 1);
+            CFB_LAUNCH();
+            CFB_TRY(fetch_counters(bt));
+            if (bt->h_counters[0] > 0)
             {
-                cudaGraphExec_t exec;
-                CFB_TRY(batch_graph(bt, order, &exec));
-                CFB_CUDA(cudaGraphLaunch(exec, s));
-            }
-            else if (!ran)
-            {
-                for (int it = 0; it < o->maxIter; ++it)
+                // opt-in: the whole inner loop of all systems as one launch
+                bool ran = false;
+                if (o->graph && o->persistentMaxCells > 0 && bt->N <= o->persistentMaxCells)
+                    CFB_TRY(persistent_loop(bt, order, &ran));
+                if (!ran && o->graph)
                 {
-                    CFB_TRY(launch_body(bt, order, 0, 0));
-                    CFB_TRY(fetch_counters(bt));
-                    if (bt->h_counters[0] <= 0) break;
+                    cudaGraphExec_t exec;
+                    CFB_TRY(batch_graph(bt, order, &exec));
+                    CFB_CUDA(cudaGraphLaunch(exec, s));
+                }
+                else if (!ran)
+                {
+                    for (int it = 0; it < o->maxIter; ++it)
+                    {
+                        CFB_TRY(launch_body(bt, order, 0, 0));
+                        CFB_TRY(fetch_counters(bt));
+                        if (bt->h_counters[0] <= 0) break;
+                    }
                 }
             }
         }
@@ -1516,6 +1795,7 @@ extern "C" int cf_batch_destroy(cf_batch* bt)
     if (!bt) return CF_OK;
     cudaSetDevice(bt->device);
     if (bt->stream) cudaStreamSynchronize(bt->stream);
+    whole_release(bt);
     for (cf_context* c : bt->solo)
         if (c) cf_context_destroy(c);
     for (auto& kv : bt->graphs) cudaGraphExecDestroy(kv.second);
@@ -1760,6 +2040,12 @@ extern "C" int cf_batch_finalize(cf_batch* bt, int32_t reorder)
     CFB_CUDA(cudaMemsetAsync(bt->d_io64, 0, sizeof(double) * N, s));
     CFB_CUDA(cudaMemsetAsync(bt->d_io64b, 0, sizeof(double) * N, s));
     CFB_CUDA(cudaStreamSynchronize(s));
+    // whole inner solves, unless systems run as solo solves beside them
+    if ((int)bt->sys.size() == bt->nAll && whole_build(bt, reorder) != CF_OK)
+    {
+        cudaGetLastError();   // no memory for the splits: the batched loop
+        whole_release(bt);
+    }
     for (auto& y : bt->sys)
     {
         std::vector<int32_t>().swap(y.L.col);   // host copies no longer needed

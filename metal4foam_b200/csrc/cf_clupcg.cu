@@ -69,8 +69,6 @@ struct CluArgs
 {
     const CluSys* list;   // the systems of the launch, or null: `one`
     CluSys one;
-    int order;
-    long long polls;
 };
 
 // Sums of v[0..NR) over the CTA, pushed to every CTA of the cluster.
@@ -149,7 +147,8 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
     const int ctas = (int)cl.num_blocks();
     const int rank = (int)cl.block_rank();
     const CluSys& Y = a.list ? a.list[blockIdx.x / ctas] : a.one;
-    if (Y.fromState && Y.st->done) return;   // (the whole cluster)
+    const InnerRun& N = Y.run;
+    if (N.fromState && N.st->done) return;   // (the whole cluster)
     const CluSplit& C = Y.split;
     const ResPart P = C.parts[rank];
     const int locP = C.locP;
@@ -157,15 +156,15 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
     float* zc = zmem;          // current z
     float* zn = zmem + zs;     // the next
     float* pb = zmem + 2 * zs;
-    const bool cheb = a.order > 1;
-    const float c1 = cheb ? __ldg(Y.chebC) : 1.0f;
-    const double mean = Y.mean && (!Y.useMean || *Y.useMean) ? *Y.mean : 0.0;
+    const bool cheb = N.order > 1;
+    const float c1 = cheb ? __ldg(N.chebC) : 1.0f;
+    const double mean = N.mean && (!N.useMean || *N.useMean) ? *N.mean : 0.0;
     if (tid == 0)
     {
-        if (Y.fromState)
-            inner_state_init(sh.S, Y.st->target, Y.st->maxIter, Y.st->ips, Y.st->stagLimit);
+        if (N.fromState)
+            inner_state_init(sh.S, N.st->target, N.st->maxIter, N.st->ips, N.st->stagLimit);
         else
-            inner_state_init(sh.S, Y.target, Y.maxIter, Y.ips, Y.stagLimit);
+            inner_state_init(sh.S, N.target, N.maxIter, N.ips, N.stagLimit);
         sh.stop = sh.bad = 0;
     }
     for (int i = tid; i < 2 * CLU_MAX_CTAS * 4; i += T) (&sh.words[0][0][0])[i] = 0;
@@ -195,14 +194,14 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
         for (int k = 0; k < W; ++k)
         {
             const int e = C.emap[pair_index(sb, W, k, l & 31)];
-            v[i][k] = e >= 0 ? Y.val32[e] : 0.0f;
+            v[i][k] = e >= 0 ? N.val32[e] : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q)
             if (q < C.ndest) dst[i][q] = C.dest[(size_t)q * C.rowsP + P.rowBase + l];
-        dg[i] = Y.diag32[g];
-        rd[i] = Y.rD32[g];
-        const float ra = (float)(Y.r64[g] - mean);
+        dg[i] = N.diag32[g];
+        rd[i] = N.rD32[g];
+        const float ra = (float)(N.r64[g] - mean);
         r[i] = ra;
         z[i] = w[i] = cheb ? __fmul_rn(__fmul_rn(c1, rd[i]), ra) : __fmul_rn(ra, rd[i]);
         if (!cheb) accZ += (double)z[i] * (double)ra;
@@ -227,7 +226,7 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
     };
     auto halo_wait = [&]() {
         const unsigned int at = smem_addr(zc + locP);
-        for (int h = tid; h < P.nh; h += T) wait_local(at + 8 * h, ep, &sh.bad, a.polls);
+        for (int h = tid; h < P.nh; h += T) wait_local(at + 8 * h, ep, &sh.bad, N.polls);
     };
     cl.sync();
 #pragma unroll
@@ -238,14 +237,14 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
     for (;;)
     {
         if (cheb) accZ = 0.0;
-        for (int j = 1; j < a.order; ++j)
+        for (int j = 1; j < N.order; ++j)
         {
-            const float c2 = __ldg(Y.chebC + 2 * j - 1);
-            const float c3 = __ldg(Y.chebC + 2 * j);
+            const float c2 = __ldg(N.chebC + 2 * j - 1);
+            const float c3 = __ldg(N.chebC + 2 * j);
             halo_wait();
             __syncthreads();
             ++ep;
-            const bool last = j == a.order - 1;
+            const bool last = j == N.order - 1;
             const unsigned int buf = smem_addr(zn + locP);
             // (rows past the part's end hold zeros and need no test)
 #pragma unroll
@@ -278,7 +277,7 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
             double acc[2] = {accR, accZ};
             clu_send<2>(acc, 0, rank, ctas, ep, sh, tid, T);
             halo_wait();
-            clu_recv<2>(0, ctas, ep, sh, tid, a.polls);
+            clu_recv<2>(0, ctas, ep, sh, tid, N.polls);
             __syncthreads();
         }
         const double zr = sh.tot[1];
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
             inner_after_apply(sh.S, first, rsum, wArA);
             sh.stop = sh.S.done || sh.bad;
         }
-        clu_recv<1>(1, ctas, ep, sh, tid, a.polls);
+        clu_recv<1>(1, ctas, ep, sh, tid, N.polls);
         __syncthreads();
         first = false;
         if (sh.stop) break;
@@ -342,13 +341,13 @@ __global__ void __launch_bounds__(CLU_T, 1) k_clu_pcg(const __grid_constant__ Cl
     }
     if (tid == T - 1)
     {
-        if (sh.bad) atomicExch(&Y.st->waitErr, 1);
-        inner_finish(sh.S, Y.st, rank == 0);
+        if (sh.bad) atomicExch(&N.st->waitErr, 1);
+        inner_finish(sh.S, N.st, rank == 0);
     }
     __syncthreads();
     const int sel = sh.S.sel;
     const float* ds = Y.dw + (size_t)sel * C.rowsP + P.rowBase;
-    float* out = Y.D + (size_t)sel * Y.dStride;
+    float* out = N.D + (size_t)sel * N.dStride;
 #pragma unroll
     for (int i = 0; i < R; ++i)
     {
@@ -395,21 +394,20 @@ struct Pack
     }
 };
 
-int config(const CluPlan* p, int count, cudaStream_t s, cudaLaunchConfig_t* cfg,
-           cudaLaunchAttribute* attr)
+void config(int ctas, int threads, size_t smem, int count, cudaStream_t s, cudaLaunchConfig_t* cfg,
+            cudaLaunchAttribute* attr)
 {
     attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = (unsigned)p->split.ctas;
+    attr->val.clusterDim.x = (unsigned)ctas;
     attr->val.clusterDim.y = 1;
     attr->val.clusterDim.z = 1;
     *cfg = {};
-    cfg->gridDim = dim3((unsigned)(p->split.ctas * count));
-    cfg->blockDim = dim3((unsigned)p->threads);
-    cfg->dynamicSmemBytes = p->smem;
+    cfg->gridDim = dim3((unsigned)(ctas * count));
+    cfg->blockDim = dim3((unsigned)threads);
+    cfg->dynamicSmemBytes = smem;
     cfg->stream = s;
     cfg->attrs = attr;
     cfg->numAttrs = 1;
-    return CF_OK;
 }
 
 }  // namespace
@@ -421,12 +419,12 @@ void clu_plan_free(CluPlan* p)
     delete p;
 }
 
-int clu_plan_build(int n, const HostLayout& L, bool ordered, int maxCtas, long long entOff,
+int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long entOff,
                    int rowOff, cudaStream_t s, CluPlan** plan)
 {
     *plan = nullptr;
     if (L.maxw > 6 || n < 1) return CF_OK;
-    const int ctas = std::max(1, std::min({maxCtas, CLU_MAX_CTAS, (n + CLU_T - 1) / CLU_T}));
+    ctas = std::max(1, std::min({ctas, CLU_MAX_CTAS, n}));
     if (n > (long long)ctas * CLU_T * CLU_MAX_R ||
         (long long)n * std::max(4, (int)L.maxw) > CLU_MAX_ENTRIES)
         return CF_OK;
@@ -495,7 +493,7 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int maxCtas, long l
     int clusters = 0;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
-    config(p, 1, s, &cfg, &attr);
+    config(ctas, p->threads, p->smem, 1, s, &cfg, &attr);
     if (p->smem > (size_t)CLU_SMEM ||
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CLU_SMEM) !=
             cudaSuccess ||
@@ -548,20 +546,18 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int maxCtas, long l
     return CF_OK;
 }
 
-int clu_launch(const CluPlan* p, const CluSys* one, const CluSys* d_list, int count, int order,
-               long long polls, cudaStream_t s)
+int clu_launch(int W, int R, int ctas, int threads, size_t smem, const CluSys* one,
+               const CluSys* d_list, int count, cudaStream_t s)
 {
     CluArgs a;
     a.list = d_list;
     if (one) a.one = *one;
     else std::memset((void*)&a.one, 0, sizeof(a.one));
-    a.order = order;
-    a.polls = polls;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
-    config(p, count, s, &cfg, &attr);
+    config(ctas, threads, smem, count, s, &cfg, &attr);
     void* args[] = {(void*)&a};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel_of(p->W, p->R), args);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel_of(W, R), args);
     if (e != cudaSuccess)
         return fail(CF_ERR_CUDA, std::string("cluster launch: ") + cudaGetErrorString(e));
     return CF_OK;
@@ -592,8 +588,9 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
         L.nnzp = c->nnzp;
         L.maxw = c->maxRowLen;
         CluPlan* plan = nullptr;
-        const int rc = clu_plan_build(c->n, L, !c->identityPerm, CLU_MAX_CTAS, 0, 0, c->stream, &plan);
-        if (rc != CF_OK) return rc;
+        const int ctas = std::min(CLU_MAX_CTAS, (c->n + CLU_T - 1) / CLU_T);
+        if (clu_plan_build(c->n, L, !c->identityPerm, ctas, 0, 0, c->stream, &plan) != CF_OK)
+            cudaGetLastError();   // no memory for the split: another path
         c->clu = plan;
     }
     CluPlan* p = static_cast<CluPlan*>(c->clu);
@@ -601,23 +598,9 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
     cudaStream_t s = c->stream;
     CluSys Y;
     Y.split = p->split;
-    Y.val32 = c->d_val32;
-    Y.diag32 = c->d_diag32;
-    Y.rD32 = c->d_rD32;
-    Y.chebC = c->d_chebC;
-    Y.r64 = c->d_r64;
-    Y.mean = mean;
-    Y.useMean = nullptr;
-    Y.D = c->d_D;
-    Y.dStride = c->n;
+    Y.run = inner_run(c, mean, target, maxIter, ips, order, stagLimit);
     Y.dw = p->dw;
-    Y.st = c->d_st;
-    Y.fromState = 0;
-    Y.target = target;
-    Y.maxIter = maxIter;
-    Y.ips = ips;
-    Y.stagLimit = stagLimit;
-    const int rc = clu_launch(p, &Y, nullptr, 1, order, c->waitPolls, s);
+    const int rc = clu_launch(p->W, p->R, p->split.ctas, p->threads, p->smem, &Y, nullptr, 1, s);
     if (rc != CF_OK) return rc;
     c->launches++;
     CLU_CUDA(cudaEventRecord(c->ev1, s));

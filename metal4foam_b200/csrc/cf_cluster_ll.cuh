@@ -38,20 +38,8 @@ struct CluSplit
 struct CluSys
 {
     CluSplit split;
-    const float* val32;
-    const float* diag32;
-    const float* rD32;
-    const float* chebC;
-    const double* r64;
-    const double* mean;           // subtracted from r64 (null: 0) ...
-    const int* useMean;           // ... when this is null or points to != 0
-    float* D;                     // [3][dStride] corrections (internal order)
-    long long dStride;
+    InnerRun run;
     float* dw;                    // [3][rowsP] corrections (part order)
-    InnerState* st;
-    int fromState;                // target, maxIter, ips, stagLimit as *st has them
-    double target;
-    int maxIter, ips, stagLimit;
 };
 
 // The device copy of a split and the kernel that runs it.
@@ -66,15 +54,15 @@ struct CluPlan
 
 struct HostLayout;
 
-// Splits a mesh for the cluster PCG (entOff: added to the entries of L when
-// its arrays are part of a larger concatenation); leaves plan null when the
-// kernel does not take the mesh.
-int clu_plan_build(int n, const HostLayout& L, bool ordered, int maxCtas, long long entOff,
+// Splits a mesh over at most `ctas` CTAs for the cluster PCG (entOff, rowOff
+// as for res_plan_build); leaves plan null when the kernel does not take it.
+int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long entOff,
                    int rowOff, cudaStream_t s, CluPlan** plan);
 void clu_plan_free(CluPlan* plan);
-// One launch over `count` systems with the same (W, R, threads, ctas, smem).
-int clu_launch(const CluPlan* p, const CluSys* one, const CluSys* d_list, int count, int order,
-               long long polls, cudaStream_t s);
+// One launch: the system `one`, or the `count` systems of d_list, whose plans
+// share W, R and the number of CTAs (threads, smem: the largest of theirs).
+int clu_launch(int W, int R, int ctas, int threads, size_t smem, const CluSys* one,
+               const CluSys* d_list, int count, cudaStream_t s);
 
 __device__ __forceinline__ unsigned int smem_addr(const void* p)
 {

@@ -270,6 +270,9 @@ int persistent_status(cf_context* c);
 // one and no other resident launch of the process runs on the device; *ran
 // tells whether it did.
 constexpr int RESIDENT_MIN_ROWS_PER_SM = 128;
+struct InnerRun;
+InnerRun inner_run(const cf_context* c, const double* mean, double target, int maxIter, int ips,
+                   int order, int stagLimit);
 int resident_build(cf_context* c, const HostLayout& L);
 void resident_release(cf_context* c);
 int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,

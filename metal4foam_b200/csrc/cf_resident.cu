@@ -70,6 +70,26 @@ using namespace cf;
 
 namespace cf {
 
+struct ResPlan
+{
+    int nparts = 0, W = 0, slots = 0, rowsP = 0, maxLocP = 0, maxHalo = 0;
+    int R = 0;                    // rows per thread
+    int TB = 0, threads = 0;
+    size_t smem = 0;
+    const void* fn = nullptr;
+    std::vector<void*> allocs;
+    ResPart* parts = nullptr;
+    int* rowMap = nullptr;
+    unsigned short* idx = nullptr;
+    int* emap = nullptr;
+    int* haloSlot = nullptr;
+    u64* ll = nullptr;
+    u64* red = nullptr;
+    unsigned int* epoch = nullptr;
+    float* dw = nullptr;
+    float* dc = nullptr;
+};
+
 namespace {
 
 constexpr int RES_MAX_PARTS = 256;   // CTAs of one system at most
@@ -90,23 +110,10 @@ struct ResArgs
     int slots;
     u64* red;                // [2][copy][part][2 values x 2 words]
     unsigned int* epoch;     // last epoch used by the launches before
-    // operator and right-hand side (internal order)
-    const float* val32;
-    const float* diag32;
-    const float* rD32;
-    const float* chebC;
-    const double* r64;
-    const double* mean;
-    // results (internal order) and work space (part order)
-    float* D;                // [3 n]
-    float* dw;               // [3 rowsP] corrections
+    float* dw;               // [3 rowsP] corrections (part order)
     float* dc;               // [rowsP] current correction of the lean kernels
     int rowsP;
-    InnerState* st;
-    int n, order;
-    double target;
-    int maxIter, ips, stagLimit;
-    long long polls;
+    InnerRun run;
 };
 
 __device__ __forceinline__ u64 ld_word(const u64* p)
@@ -211,11 +218,11 @@ __device__ __forceinline__ void halo_recv(const ResArgs& a, const ResPart& P, co
     for (int q = 0; q < RES_HQ; ++q)
         if (hs[q] >= 0)
             x[P.nlocP + tid + q * T] =
-                __uint_as_float(wait_word(ll + hs[q], v[q], epoch, sh, a.st, a.polls));
+                __uint_as_float(wait_word(ll + hs[q], v[q], epoch, sh, a.run.st, a.run.polls));
     for (int h = tid + RES_HQ * T; h < P.nh; h += T)
     {
         const u64* p = ll + __ldg(a.haloSlot + P.haloBase + h);
-        x[P.nlocP + h] = __uint_as_float(wait_word(p, ld_word(p), epoch, sh, a.st, a.polls));
+        x[P.nlocP + h] = __uint_as_float(wait_word(p, ld_word(p), epoch, sh, a.run.st, a.run.polls));
     }
 }
 
@@ -273,7 +280,7 @@ __device__ __forceinline__ void red_recv(const ResArgs& a, const u64* red, int r
 #pragma unroll
         for (int r = 0; r < NR; ++r)
         {
-            acc[r] += wait_double(w + 2 * r, f[r][0], f[r][1], epoch, sh, a.st, a.polls);
+            acc[r] += wait_double(w + 2 * r, f[r][0], f[r][1], epoch, sh, a.run.st, a.run.polls);
         }
     }
 #pragma unroll
@@ -294,7 +301,11 @@ __device__ __forceinline__ double red_total(const ResArgs& a, const ResShared& s
 
 __device__ __forceinline__ void state_init(const ResArgs& a, ResShared& sh)
 {
-    inner_state_init(sh.S, a.target, a.maxIter, a.ips, a.stagLimit);
+    const InnerState* s = a.run.st;
+    if (a.run.fromState)
+        inner_state_init(sh.S, s->target, s->maxIter, s->ips, s->stagLimit);
+    else
+        inner_state_init(sh.S, a.run.target, a.run.maxIter, a.run.ips, a.run.stagLimit);
     sh.stop = 0;
     sh.bad = 0;
 }
@@ -311,6 +322,7 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
 {
     extern __shared__ float zmem[];
     __shared__ ResShared sh;
+    if (a.run.fromState && a.run.st->done) return;   // (the whole grid)
     constexpr bool LEAN = R * TB > 2560;   // z, delta and q of a row are not kept in registers
     // Rows of the first RB thread rows are finished and published one after
     // the other, the rest (rows no other part reads, mostly) in whatever
@@ -332,9 +344,10 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
     const int mRows = max(0, P.nlocP - m0);
     float* sval = zmem + ((3 * zs + 1) & ~1);
     unsigned short* sidx = reinterpret_cast<unsigned short*>(sval + (size_t)mRows * W);
-    const bool cheb = a.order > 1;
-    const float c1 = cheb ? __ldg(a.chebC) : 1.0f;
-    const double mean = a.mean ? *a.mean : 0.0;
+    const bool cheb = a.run.order > 1;
+    const float c1 = cheb ? __ldg(a.run.chebC) : 1.0f;
+    const double mean =
+        a.run.mean && (!a.run.useMean || *a.run.useMean) ? *a.run.mean : 0.0;
     unsigned int ep = *(volatile unsigned int*)a.epoch;
     if (tid == 0)
     {
@@ -384,7 +397,7 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
                 for (int k = 0; k < W; ++k)
                 {
                     const int e = a.emap[pair_index(sb, W, k, l & 31)];
-                    v[i < RM ? i : 0][k] = e >= 0 ? a.val32[e] : 0.0f;
+                    v[i < RM ? i : 0][k] = e >= 0 ? a.run.val32[e] : 0.0f;
                 }
             }
         }
@@ -396,14 +409,14 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
             {
                 const int o = (int)pair_index(0, W, k, l & 31);
                 const int e = a.emap[sb + o];
-                sval[at0 + o] = e >= 0 ? a.val32[e] : 0.0f;
+                sval[at0 + o] = e >= 0 ? a.run.val32[e] : 0.0f;
                 sidx[at0 + o] = a.idx[sb + o];
             }
         }
         if (g < 0) continue;
-        dg[i] = a.diag32[g];
-        rd[i] = a.rD32[g];
-        const float ra = (float)(a.r64[g] - mean);
+        dg[i] = a.run.diag32[g];
+        rd[i] = a.run.rD32[g];
+        const float ra = (float)(a.run.r64[g] - mean);
         r[i] = ra;
         const float z0 = cheb ? __fmul_rn(__fmul_rn(c1, rd[i]), ra) : __fmul_rn(ra, rd[i]);
         w[i] = z0;
@@ -446,14 +459,14 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
     for (;;)
     {
         if (cheb) accZ = 0.0;
-        for (int j = 1; j < a.order; ++j)
+        for (int j = 1; j < a.run.order; ++j)
         {
-            const float c2 = __ldg(a.chebC + 2 * j - 1);
-            const float c3 = __ldg(a.chebC + 2 * j);
+            const float c2 = __ldg(a.run.chebC + 2 * j - 1);
+            const float c3 = __ldg(a.run.chebC + 2 * j);
             halo_recv(a, P, hs, lr, ep, zc, sh, tid, T);
             __syncthreads();
             ++ep;
-            const bool last = j == a.order - 1;
+            const bool last = j == a.run.order - 1;
             if constexpr (!LEAN)
             {
                 // (rows past the part's end hold zeros and need no test)
@@ -615,11 +628,11 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
         }
         swap_ptr(lw, lr);
     }
-    if (tid == T - 1) inner_finish(sh.S, a.st, rank == 0);
+    if (tid == T - 1) inner_finish(sh.S, a.run.st, rank == 0);
     __syncthreads();
     const int sel = sh.S.sel;
     const float* ds = a.dw + (size_t)sel * a.rowsP + P.rowBase;
-    float* out = a.D + (size_t)sel * a.n;
+    float* out = a.run.D + (size_t)sel * a.run.dStride;
 #pragma unroll
     for (int i = 0; i < R; ++i)
     {
@@ -632,28 +645,6 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
 
 // ------------------------------------------------------------------- host
 
-struct ResPlan
-{
-    int nparts = 0, W = 0, slots = 0, rowsP = 0, maxLocP = 0, maxHalo = 0;
-    int R = 0;                    // rows per thread
-    int TB = 0, threads = 0;
-    size_t smem = 0;
-    const void* fn = nullptr;
-    std::vector<void*> allocs;
-    ResPart* parts = nullptr;
-    int* rowMap = nullptr;
-    unsigned short* idx = nullptr;
-    int* emap = nullptr;
-    int* haloSlot = nullptr;
-    u64* ll = nullptr;
-    u64* red = nullptr;
-    unsigned int* epoch = nullptr;
-    float* dw = nullptr;
-    float* dc = nullptr;
-};
-
-// The CTAs of a resident launch wait for one another, so one launch at a
-// time per device: a solve that finds the device taken runs the graph path.
 std::mutex g_resident[64];
 
 // The kernels: R rows per thread, RM of them with their matrix entries in
@@ -679,59 +670,71 @@ const ChipKernel CHIP[] = {
     RES_CHIP(10, 5, 512), RES_CHIP(12, 5, 512)};
 
 template <class T>
-int up(cf_context* c, ResPlan* p, T** d, const T* h, size_t count)
+int up(ResPlan* p, T** d, const T* h, size_t count, cudaStream_t s)
 {
     RES_CUDA(cudaMalloc((void**)d, std::max<size_t>(count, 1) * sizeof(T)));
     p->allocs.push_back((void*)*d);
     if (h && count)
-        RES_CUDA(cudaMemcpyAsync(*d, h, count * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+        RES_CUDA(cudaMemcpyAsync(*d, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
     return CF_OK;
 }
 
 }  // namespace
 
-void resident_release(cf_context* c)
+std::mutex& res_device_lock(int device) { return g_resident[device & 63]; }
+
+void res_plan_free(ResPlan* p)
 {
-    ResPlan* p = static_cast<ResPlan*>(c->resident);
     if (!p) return;
     for (void* q : p->allocs) cudaFree(q);
     delete p;
-    c->resident = nullptr;
 }
 
-int resident_build(cf_context* c, const HostLayout& L)
+int res_reset(const ResPlan* p, cudaStream_t s)
 {
-    resident_release(c);
-    const int nparts = std::min(c->numSMs, RES_MAX_PARTS);
-    if (!c->coopLaunch || c->n < RESIDENT_MIN_ROWS_PER_SM * nparts || L.maxw < 4 || L.maxw > 6 ||
-        c->n > (long long)nparts * RES_MAX_ROWS || c->device >= 64)
+    RES_CUDA(cudaMemsetAsync(p->ll, 0, sizeof(u64) * 2 * (size_t)std::max(p->slots, 1), s));
+    RES_CUDA(cudaMemsetAsync(p->red, 0, sizeof(u64) * 2 * RES_RED_WORDS, s));
+    RES_CUDA(cudaMemsetAsync(p->epoch, 0, sizeof(unsigned int), s));
+    return CF_OK;
+}
+
+int res_plan_build(int device, int n, const HostLayout& L, bool ordered, int nparts,
+                   long long entOff, int rowOff, cudaStream_t s, ResPlan** plan)
+{
+    *plan = nullptr;
+    if (L.maxw > 6 || nparts < 1 || nparts > RES_MAX_PARTS ||
+        n > (long long)nparts * RES_MAX_ROWS)
         return CF_OK;
     ResHost H;
     ResPlan* p = nullptr;
     try
     {
-        if (!res_partition(c->n, L, !c->identityPerm, nparts, H)) return CF_OK;
+        if (!res_partition(n, L, ordered, nparts, H, 4)) return CF_OK;
+        if (entOff)
+            for (int32_t& e : H.emap)
+                if (e >= 0) e += (int32_t)entOff;
+        if (rowOff)
+            for (int32_t& r : H.rowMap)
+                if (r >= 0) r += rowOff;
         p = new ResPlan();
     }
     catch (...)
     {
-        return CF_OK;   // no memory for the split: the graph path
+        return CF_OK;   // no memory for the split
     }
-    c->resident = p;
     p->nparts = nparts;
     p->W = H.W;
     p->slots = H.slots;
     p->rowsP = H.rowsP;
-    p->maxLocP = H.maxLocP;
-    p->maxHalo = H.maxHalo;
     int maxSmem = 0;
-    RES_CUDA(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    if (cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) !=
+        cudaSuccess)
+        maxSmem = 0;
     // z (two buffers) and p; the parts differ in their halo, so the largest
     size_t zf = 0;
     for (const ResPart& q : H.parts) zf = std::max(zf, (size_t)3 * (q.nlocP + q.nh + 1) + 1);
     const size_t zbytes = sizeof(float) * ((zf + 1) & ~(size_t)1);
-    const size_t avail = (size_t)maxSmem - 2048;   // static shared state
-    p->R = 0;
+    const size_t avail = (size_t)std::max(maxSmem - 2048, 0);   // static shared state
     for (const ChipKernel& k : CHIP)
     {
         if (H.maxLocP > k.R * k.TB) continue;
@@ -746,56 +749,45 @@ int resident_build(cf_context* c, const HostLayout& L)
         p->fn = k.fn[H.W - 4];
         break;
     }
-    if (!p->fn)
-    {
-        resident_release(c);
-        return CF_OK;
-    }
-    // one value for every context of the process: a solve on another thread
-    // never lowers it under a launch
-    if (cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail) !=
-        cudaSuccess)
-    {
-        cudaGetLastError();
-        resident_release(c);
-        return CF_OK;
-    }
+    // (the attribute: one value for every context of the process, so a solve
+    // on another thread never lowers it under a launch)
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p->fn, p->threads, p->smem) !=
+    if (!p->fn ||
+        cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)avail) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, p->fn, p->threads, p->smem) !=
             cudaSuccess ||
         occ < 1)
     {
         cudaGetLastError();
-        resident_release(c);
+        res_plan_free(p);
         return CF_OK;
     }
-    int rc = up(c, p, &p->parts, H.parts.data(), H.parts.size());
-    if (rc == CF_OK) rc = up(c, p, &p->rowMap, H.rowMap.data(), H.rowMap.size());
-    if (rc == CF_OK) rc = up(c, p, &p->idx, (const unsigned short*)H.idx.data(), H.idx.size());
-    if (rc == CF_OK) rc = up(c, p, &p->emap, H.emap.data(), H.emap.size());
-    if (rc == CF_OK) rc = up(c, p, &p->haloSlot, H.haloSlot.data(), H.haloSlot.size());
-    if (rc == CF_OK) rc = up<u64>(c, p, &p->ll, nullptr, 2 * (size_t)H.slots);
-    if (rc == CF_OK) rc = up<u64>(c, p, &p->red, nullptr, 2 * RES_RED_WORDS);
-    if (rc == CF_OK) rc = up<unsigned int>(c, p, &p->epoch, nullptr, 1);
-    if (rc == CF_OK) rc = up<float>(c, p, &p->dw, nullptr, 3 * (size_t)H.rowsP);
-    if (rc == CF_OK && p->R * p->TB > 2560) rc = up<float>(c, p, &p->dc, nullptr, (size_t)H.rowsP);
-    if (rc != CF_OK) return rc;
-    RES_CUDA(cudaMemsetAsync(p->ll, 0, sizeof(u64) * 2 * (size_t)std::max(H.slots, 1), c->stream));
-    RES_CUDA(cudaMemsetAsync(p->red, 0, sizeof(u64) * 2 * RES_RED_WORDS, c->stream));
-    RES_CUDA(cudaMemsetAsync(p->epoch, 0, sizeof(unsigned int), c->stream));
-    RES_CUDA(cudaStreamSynchronize(c->stream));   // the host arrays end here
+    int rc = up(p, &p->parts, H.parts.data(), H.parts.size(), s);
+    if (rc == CF_OK) rc = up(p, &p->rowMap, H.rowMap.data(), H.rowMap.size(), s);
+    if (rc == CF_OK) rc = up(p, &p->idx, (const unsigned short*)H.idx.data(), H.idx.size(), s);
+    if (rc == CF_OK) rc = up(p, &p->emap, H.emap.data(), H.emap.size(), s);
+    if (rc == CF_OK) rc = up(p, &p->haloSlot, H.haloSlot.data(), H.haloSlot.size(), s);
+    if (rc == CF_OK) rc = up<u64>(p, &p->ll, nullptr, 2 * (size_t)H.slots, s);
+    if (rc == CF_OK) rc = up<u64>(p, &p->red, nullptr, 2 * RES_RED_WORDS, s);
+    if (rc == CF_OK) rc = up<unsigned int>(p, &p->epoch, nullptr, 1, s);
+    if (rc == CF_OK) rc = up<float>(p, &p->dw, nullptr, 3 * (size_t)H.rowsP, s);
+    if (rc == CF_OK && p->R * p->TB > 2560)
+        rc = up<float>(p, &p->dc, nullptr, (size_t)H.rowsP, s);
+    if (rc == CF_OK) rc = res_reset(p, s);
+    if (rc == CF_OK && cudaStreamSynchronize(s) != cudaSuccess)   // the host arrays end here
+        rc = fail(CF_ERR_CUDA, "split over the SMs: upload");
+    if (rc != CF_OK)
+    {
+        res_plan_free(p);
+        return rc;
+    }
+    *plan = p;
     return CF_OK;
 }
 
-int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,
-                   int order, int stagLimit, bool* ran)
+int res_launch(const ResPlan* p, const InnerRun& run, cudaStream_t s)
 {
-    *ran = false;
-    ResPlan* p = static_cast<ResPlan*>(c->resident);
-    if (!p || maxIter <= 0) return CF_OK;
-    std::unique_lock<std::mutex> turn(g_resident[c->device], std::try_to_lock);
-    if (!turn.owns_lock()) return CF_OK;
-    cudaStream_t s = c->stream;
     ResArgs a;
     a.parts = p->parts;
     a.nparts = p->nparts;
@@ -807,29 +799,73 @@ int resident_inner(cf_context* c, const double* mean, double target, int maxIter
     a.slots = p->slots;
     a.red = p->red;
     a.epoch = p->epoch;
-    a.val32 = c->d_val32;
-    a.diag32 = c->d_diag32;
-    a.rD32 = c->d_rD32;
-    a.chebC = c->d_chebC;
-    a.r64 = c->d_r64;
-    a.mean = mean;
-    a.D = c->d_D;
     a.dw = p->dw;
     a.dc = p->dc;
     a.rowsP = p->rowsP;
-    a.st = c->d_st;
-    a.n = c->n;
-    a.order = order;
-    a.target = target;
-    a.maxIter = maxIter;
-    a.ips = ips;
-    a.stagLimit = stagLimit;
-    a.polls = std::min(c->waitPolls, 1LL << 22);
+    a.run = run;
+    a.run.polls = std::min(run.polls, 1LL << 22);
     void* args[] = {(void*)&a};
     const cudaError_t e = cudaLaunchCooperativeKernel(p->fn, dim3(p->nparts), dim3(p->threads),
                                                       args, p->smem, s);
     if (e != cudaSuccess)
         return fail(CF_ERR_CUDA, std::string("cudaLaunchCooperativeKernel: ") + cudaGetErrorString(e));
+    return CF_OK;
+}
+
+InnerRun inner_run(const cf_context* c, const double* mean, double target, int maxIter, int ips,
+                   int order, int stagLimit)
+{
+    InnerRun r;
+    r.val32 = c->d_val32;
+    r.diag32 = c->d_diag32;
+    r.rD32 = c->d_rD32;
+    r.chebC = c->d_chebC;
+    r.r64 = c->d_r64;
+    r.mean = mean;
+    r.useMean = nullptr;
+    r.D = c->d_D;
+    r.dStride = c->n;
+    r.st = c->d_st;
+    r.fromState = 0;
+    r.order = order;
+    r.target = target;
+    r.maxIter = maxIter;
+    r.ips = ips;
+    r.stagLimit = stagLimit;
+    r.polls = c->waitPolls;
+    return r;
+}
+
+void resident_release(cf_context* c)
+{
+    res_plan_free(static_cast<ResPlan*>(c->resident));
+    c->resident = nullptr;
+}
+
+int resident_build(cf_context* c, const HostLayout& L)
+{
+    resident_release(c);
+    const int nparts = std::min(c->numSMs, RES_MAX_PARTS);
+    if (!c->coopLaunch || c->n < RESIDENT_MIN_ROWS_PER_SM * nparts || L.maxw < 4) return CF_OK;
+    ResPlan* p = nullptr;
+    if (res_plan_build(c->device, c->n, L, !c->identityPerm, nparts, 0, 0, c->stream, &p) != CF_OK)
+        cudaGetLastError();   // no memory for the split: the graph path
+    c->resident = p;
+    return CF_OK;
+}
+
+int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,
+                   int order, int stagLimit, bool* ran)
+{
+    *ran = false;
+    const ResPlan* p = static_cast<const ResPlan*>(c->resident);
+    if (!p || maxIter <= 0) return CF_OK;
+    // (another resident launch on the device: the graph path)
+    std::unique_lock<std::mutex> turn(res_device_lock(c->device), std::try_to_lock);
+    if (!turn.owns_lock()) return CF_OK;
+    cudaStream_t s = c->stream;
+    const int rc = res_launch(p, inner_run(c, mean, target, maxIter, ips, order, stagLimit), s);
+    if (rc != CF_OK) return rc;
     c->launches++;
     // the device is taken until the launch has ended
     RES_CUDA(cudaEventRecord(c->ev1, s));
@@ -837,11 +873,9 @@ int resident_inner(cf_context* c, const double* mean, double target, int maxIter
     RES_CUDA(cudaStreamSynchronize(s));
     if (c->h_st->waitErr)
     {
-        // a wait gave up: fresh words for the next launch, this solve goes
-        // through the graph path
-        RES_CUDA(cudaMemsetAsync(p->ll, 0, sizeof(u64) * 2 * (size_t)std::max(p->slots, 1), s));
-        RES_CUDA(cudaMemsetAsync(p->red, 0, sizeof(u64) * 2 * RES_RED_WORDS, s));
-        RES_CUDA(cudaMemsetAsync(p->epoch, 0, sizeof(unsigned int), s));
+        // a wait gave up: this solve goes through the graph path
+        const int rr = res_reset(p, s);
+        if (rr != CF_OK) return rr;
         RES_CUDA(cudaMemsetAsync(&c->d_st->waitErr, 0, sizeof(int), s));
         return CF_OK;
     }

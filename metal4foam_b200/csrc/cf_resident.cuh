@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <vector>
 
 #include "cf_internal.cuh"
@@ -40,6 +41,42 @@ struct ResHost
     std::vector<int32_t> emap;        // [rowsP * W] entry of the SELL arrays, -1 padding
     std::vector<int32_t> haloSlot;    // exchange slot of every halo value
 };
+
+// One inner PCG on the staged FP32 operator, as the kernels that run it whole
+// take it (everything in the internal row order).
+struct InnerRun
+{
+    const float* val32;
+    const float* diag32;
+    const float* rD32;
+    const float* chebC;
+    const double* r64;
+    const double* mean;           // subtracted from r64 (null: 0) ...
+    const int* useMean;           // ... when this is null or points to != 0
+    float* D;                     // [3][dStride] corrections
+    long long dStride;
+    InnerState* st;
+    int fromState;                // target, maxIter, ips, stagLimit (and done) as *st has them
+    int order;
+    double target;
+    int maxIter, ips, stagLimit;
+    long long polls;              // reads a bounded wait makes before it gives up
+};
+
+// The mesh split over the CTAs of one cooperative launch (cf_resident.cu).
+// entOff, rowOff: where the entries and rows of L start when its arrays are
+// part of a larger concatenation.  *plan stays null when no kernel takes the
+// mesh.
+struct ResPlan;
+int res_plan_build(int device, int n, const HostLayout& L, bool ordered, int nparts,
+                   long long entOff, int rowOff, cudaStream_t s, ResPlan** plan);
+void res_plan_free(ResPlan* plan);
+// The waits of a resident launch need all its CTAs on the device: launches
+// run under this lock, with at most one CTA per SM in all.
+std::mutex& res_device_lock(int device);
+int res_launch(const ResPlan* plan, const InnerRun& run, cudaStream_t s);
+// fresh exchange words after a wait has given up
+int res_reset(const ResPlan* plan, cudaStream_t s);
 
 // Splits the rows of L (its internal order; `ordered`: reverse
 // Cuthill-McKee) into nparts parts of equal size (within one row).  Returns

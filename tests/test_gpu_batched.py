@@ -205,3 +205,36 @@ def test_batch_solo_systems(require_gpu):
         assert p.converged and p.finalResidual < 1e-6
     bt.close()
     ref.close()
+
+
+def test_batch_whole_inner_solves(require_gpu):
+    """Without solo systems every inner solve runs whole: as clusters (one
+    launch for the systems with the same kernel) or, above one cluster, as
+    cooperative launches on shares of the SMs (more systems than shares here),
+    bit for bit what the batched loop (clusterMaxCells < 0) gives."""
+    systems = small_systems() + [mesh.poisson2d(230, 190, seed=11),
+                                 mesh.varcoeff3d((40, 35, 30), seed=12, permute=True),
+                                 mesh.prism3d((40, 38, 30), seed=13),
+                                 mesh.poisson2d(330, 320, seed=14),
+                                 mesh.poisson2d(300, 310, seed=15),
+                                 mesh.varcoeff3d((46, 44, 50), seed=16, permute=False)]
+    src = [s.source for s in systems]
+    bt = make_batch(systems)
+    for kw in (dict(), dict(chebyshevOrder=1, maxIter=4000), dict(chebyshevOrder=4, deflate="off"),
+               dict(maxIter=11, maxRestarts=2)):
+        base = dict(maxRestarts=6, maxIter=3000)
+        base.update(kw)
+        a = [np.zeros(s.n) for s in systems]
+        l0 = bt.kernel_launches()
+        pa = bt.solve(a, src, _lib.default_options(clusterMaxCells=-1, **base))
+        la = bt.kernel_launches() - l0
+        b = [np.zeros(s.n) for s in systems]
+        pb = bt.solve(b, src, _lib.default_options(**base))
+        lb = bt.kernel_launches() - l0 - la
+        assert lb <= 40 * (max(p.nRestarts for p in pb) + 2), lb
+        for s, x, y, p, q in zip(systems, a, b, pa, pb):
+            assert np.array_equal(x, y), (s.name, kw)
+            for f in ("nIterations", "nRestarts", "finalResidual", "converged", "deflated",
+                      "singular", "stagnated", "polished"):
+                assert getattr(p, f) == getattr(q, f), (s.name, f)
+    bt.close()
