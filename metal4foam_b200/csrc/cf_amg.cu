@@ -466,9 +466,12 @@ struct StartX
     }
 };
 
-// Chebyshev step j >= 1:  w = c2 w + c3 rD (b - A xin);  xout = xin + w.
-// j = 0 starts the post-smoother from xin:  w = c1 rD (b - A xin).
-template <int MAXW, bool PROLONG>
+// Level 0, from the prolonged iterate: Chebyshev step j >= 1:  w = c2 w + c3 rD
+// (b - A xin);  xout = xin + w.  j = 0 starts the post-smoother:
+// w = c1 rD (b - A xin).  Level 0 reads the paired stream of its width and the
+// kernels without a sum run one row per thread, as in the Chebyshev loop:
+// 128^3 407 -> 376 us per iteration, 512^2 110 -> 102.
+template <int MAXW, int PAIRED = 0>
 __global__ void __launch_bounds__(NT) ka_step(DevSell A, const float* __restrict__ diag,
                                               const float* __restrict__ rD,
                                               const float* __restrict__ b, const float* xin,
@@ -480,11 +483,11 @@ __global__ void __launch_bounds__(NT) ka_step(DevSell A, const float* __restrict
     if (st->done) return;
     const float c2 = j > 0 ? cc[2 * j - 1] : 0.0f;
     const float c3 = j > 0 ? cc[2 * j] : cc[0];
-    const StartX<PROLONG> xf{xin, agg, xc, PROLONG ? *scale : 0.0f};
+    const StartX<true> xf{xin, agg, xc, *scale};
     CF_ROWS(row, A.n)
     {
         const float xr = xf(row);
-        const float v = row_f32<MAXW>(A, row, __fmul_rn(diag[row], xr), xf);
+        const float v = row_f32<MAXW, PAIRED>(A, row, __fmul_rn(diag[row], xr), xf);
         const float s = __fmul_rn(__fmul_rn(c3, rD[row]), __fsub_rn(b[row], v));
         const float wn = j > 0 ? __fadd_rn(__fmul_rn(c2, w[row]), s) : s;
         w[row] = wn;
@@ -493,7 +496,7 @@ __global__ void __launch_bounds__(NT) ka_step(DevSell A, const float* __restrict
 }
 
 // r = b - A x
-template <int MAXW>
+template <int MAXW, int PAIRED = 0>
 __global__ void __launch_bounds__(NT) ka_resid(DevSell A, const float* __restrict__ diag,
                                                const float* __restrict__ b,
                                                const float* __restrict__ x, float* __restrict__ r,
@@ -502,8 +505,8 @@ __global__ void __launch_bounds__(NT) ka_resid(DevSell A, const float* __restric
     if (st->done) return;
     CF_ROWS(row, A.n)
     {
-        const float v = row_f32<MAXW>(A, row, __fmul_rn(diag[row], x[row]),
-                                      [&](int q) { return __ldg(x + q); });
+        const float v = row_f32<MAXW, PAIRED>(A, row, __fmul_rn(diag[row], x[row]),
+                                              [&](int q) { return __ldg(x + q); });
         r[row] = __fsub_rn(b[row], v);
     }
 }
@@ -966,7 +969,7 @@ int launch_amg_body(cf_context* c, int degree, cudaGraphConditionalHandle h, int
     int zi = 0;
     for (int j = 1; j < degree; ++j)
     {
-        auto fn = k_cheb_step<false, MW>;
+        auto fn = cheb_step_kernel<false>(A);
         fn<<<rows_grid(c->n), NT, 0, s>>>(A, B, xa, j == 1 ? B.W0 : B.W1, B.W1, Z[zi], j, c->d_st,
                                           c->d_part);
         AMG_LAUNCH();
@@ -975,9 +978,11 @@ int launch_amg_body(cf_context* c, int degree, cudaGraphConditionalHandle h, int
     }
     float* x0 = const_cast<float*>(xa);
     // coarse-grid correction (the residual in Q, free until the p-update SpMV)
-    ka_resid<MW><<<grid_for(c, (const void*)ka_resid<MW>, c->n), NT, 0, s>>>(
-        A, B.diag, B.rA, x0, B.Q, c->d_st);
-    AMG_LAUNCH();
+    {
+        auto fn = CF_PAIRED_KERNEL(A, ka_resid, MW);
+        fn<<<rows_grid(c->n), NT, 0, s>>>(A, B.diag, B.rA, x0, B.Q, c->d_st);
+        AMG_LAUNCH();
+    }
     const AmgLevel& L0 = d->lv[0];
     float* xc = nullptr;
     // coarse levels smooth with degree 2: their Galerkin rows are wide, and
@@ -987,21 +992,24 @@ int launch_amg_body(cf_context* c, int degree, cudaGraphConditionalHandle h, int
     // level 0 post-smoothing from x + a P x'; the last step forms z.r and beta
     float* xin = x0;
     float* xout = (x0 == Z[0]) ? Z[1] : Z[0];
-    ka_step<MW, true><<<grid_for(c, (const void*)ka_step<MW, true>, c->n), NT, 0, s>>>(
-        A, B.diag, B.rD, B.rA, xin, L0.agg, xc, d->scale, B.W1, xout, c->d_chebC, 0, c->d_st);
-    AMG_LAUNCH();
+    {
+        auto fn = CF_PAIRED_KERNEL(A, ka_step, MW);
+        fn<<<rows_grid(c->n), NT, 0, s>>>(A, B.diag, B.rD, B.rA, xin, L0.agg, xc, d->scale, B.W1,
+                                          xout, c->d_chebC, 0, c->d_st);
+        AMG_LAUNCH();
+    }
     std::swap(xin, xout);
     for (int j = 1; j < degree; ++j)
     {
         if (j == degree - 1)
         {
-            auto fn = k_cheb_step<true, MW>;
+            auto fn = cheb_step_kernel<true>(A);
             fn<<<grid_for(c, (const void*)fn, c->n), NT, 0, s>>>(A, B, xin, B.W1, B.W1, xout, j,
                                                                 c->d_st, c->d_part);
         }
         else
         {
-            auto fn = k_cheb_step<false, MW>;
+            auto fn = cheb_step_kernel<false>(A);
             fn<<<rows_grid(c->n), NT, 0, s>>>(A, B, xin, B.W1, B.W1, xout, j, c->d_st, c->d_part);
         }
         AMG_LAUNCH();
@@ -1009,7 +1017,7 @@ int launch_amg_body(cf_context* c, int degree, cudaGraphConditionalHandle h, int
     }
     const float* z = xin;
     {
-        auto fn = k_pcg_p_spmv<MW>;
+        auto fn = pcg_p_spmv_kernel(A);
         fn<<<grid_for(c, (const void*)fn, c->n), NT, 0, s>>>(A, B, z, c->d_st, c->d_part);
         AMG_LAUNCH();
     }

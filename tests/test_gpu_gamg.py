@@ -285,3 +285,26 @@ def test_gamg_with_driver_controls(require_gpu):
                                                           maxIter=5000, **base))
     assert p2.converged and p2.nIterations >= p1.nIterations
     ctx.close()
+
+
+@pytest.mark.parametrize("make", [lambda: mesh.poisson2d(300, 260, seed=41),
+                                  lambda: mesh.prism3d((33, 31, 40), seed=42),
+                                  lambda: mesh.varcoeff3d((45, 41, 39), seed=43, permute=True)],
+                         ids=["w4", "w5", "w6"])
+def test_gamg_identical_with_either_stream(require_gpu, make):
+    """Level 0 on the paired stream of its slice width and on the
+    column-major 32-bit stream: the same solve bit for bit."""
+    s = make()
+    ctx = _lib.Context(0)
+    ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
+    ctx.set_coeffs(s.diag, s.upper, None)
+    out = []
+    for bits in (16, 32):
+        ctx.set_spmv_config(indexBits=bits)
+        x = np.zeros(s.n)
+        p = ctx.solve(_lib.CF_SOLVER_PCG, x, s.source,
+                      _lib.default_options(preconditioner="GAMG", tolerance=1e-8))
+        assert p.converged
+        out.append((x, p.nIterations, p.finalResidual))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
+    ctx.close()
