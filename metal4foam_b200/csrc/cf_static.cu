@@ -18,6 +18,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 
@@ -29,7 +30,8 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr int kMaxGroups = 65536;                 // partial sums (one per block)
-constexpr int kTicketSlot = kMaxGroups;           // completion counter lives here
+constexpr int kTicketSlot = kMaxGroups;           // completion counters live here
+constexpr int kTickets = 64;                      // one 256-byte line of them
 constexpr int kScratchDoubles = kMaxGroups + 32;  // + one 256-byte line for the counter
 
 // The scratch array.  Host code must not pass this name to a kernel: on the
@@ -87,12 +89,24 @@ int current_context(void** out)
 // capturing is refused with a message saying so.
 int scratch_for_current_context(cudaStream_t s, double** out)
 {
+    // the usual call: a context that has looked the address up before
+    void* ctx = nullptr;
+    if (current_context(&ctx) == CF_OK)
+    {
+        std::lock_guard<std::mutex> lock(g_scratchMutex);
+        for (int i = 0; i < g_scratchCount; ++i)
+            if (g_scratch[i].ctx == ctx)
+            {
+                *out = g_scratch[i].ptr;
+                return CF_OK;
+            }
+    }
     // the capture query also initialises the runtime (and the primary
     // context) on a thread whose first CUDA call this is
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     const cudaError_t ce = cudaStreamIsCapturing(s, &cs);
     if (ce != cudaSuccess) cudaGetLastError();
-    void* ctx = nullptr;
+    ctx = nullptr;
     int rc = current_context(&ctx);
     if (rc != CF_OK) return rc;
     std::lock_guard<std::mutex> lock(g_scratchMutex);
@@ -147,13 +161,23 @@ __device__ __forceinline__ double block_sum(double v, double* sh)
 // neighbour-side faces in losort order; separately rounded products and
 // sums) and dot = sum w.y: one partial per block in scratch, the last block
 // to finish folds them in block order.
+//
+// Bound by latency: a row's entries hang on chains of dependent loads (face
+// range -> face -> column -> x).  The first kSide faces of either side are
+// loaded level by level, all of a level together, so a row waits for four
+// trips instead of for three per face; hexahedral cells have at most three
+// faces on a side.  Products are added in the reference's order whatever the
+// order of the loads.
+constexpr int kSide = 3;
+
 __global__ void __launch_bounds__(kBlock)
     k_ldu_spmv_dot_noalloc(int n, const float* __restrict__ diag, const float* __restrict__ upper,
                            const float* __restrict__ lower, const int* __restrict__ low,
                            const int* __restrict__ upp, const int* __restrict__ ownStart,
                            const int* __restrict__ losort, const int* __restrict__ losortStart,
                            const float* __restrict__ x, const float* __restrict__ w,
-                           float* __restrict__ y, double* dot, double* scratch)
+                           float* __restrict__ y, double* dot, double* scratch,
+                           unsigned int* ticket)
 {
     __shared__ double sh[kBlock / 32];
     __shared__ bool amLast;
@@ -161,20 +185,50 @@ __global__ void __launch_bounds__(kBlock)
     double acc = 0.0;
     if (i < n)
     {
-        float sum = __fmul_rn(diag[i], x[i]);
-        for (int f = ownStart[i]; f < ownStart[i + 1]; ++f)
+        const int f0 = ownStart[i], f1 = ownStart[i + 1];
+        const int k0 = losortStart[i], k1 = losortStart[i + 1];
+        const float d = diag[i];
+        const float xi = x[i];
+        const float wi = w ? w[i] : 0.0f;
+        int oc[kSide], nf[kSide], nc[kSide];
+        float ou[kSide], ox[kSide], nl[kSide], nx[kSide];
+#pragma unroll
+        for (int q = 0; q < kSide; ++q)
+        {
+            const bool on = f0 + q < f1;
+            oc[q] = on ? upp[f0 + q] : 0;
+            ou[q] = on ? upper[f0 + q] : 0.0f;
+            nf[q] = k0 + q < k1 ? losort[k0 + q] : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < kSide; ++q)
+        {
+            const bool on = k0 + q < k1;
+            nc[q] = on ? low[nf[q]] : 0;
+            nl[q] = on ? lower[nf[q]] : 0.0f;
+            ox[q] = f0 + q < f1 ? x[oc[q]] : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < kSide; ++q) nx[q] = k0 + q < k1 ? x[nc[q]] : 0.0f;
+        float sum = __fmul_rn(d, xi);
+#pragma unroll
+        for (int q = 0; q < kSide; ++q)
+            if (f0 + q < f1) sum = __fadd_rn(sum, __fmul_rn(ou[q], ox[q]));
+        for (int f = f0 + kSide; f < f1; ++f)
             sum = __fadd_rn(sum, __fmul_rn(upper[f], x[upp[f]]));
-        for (int k = losortStart[i]; k < losortStart[i + 1]; ++k)
+#pragma unroll
+        for (int q = 0; q < kSide; ++q)
+            if (k0 + q < k1) sum = __fadd_rn(sum, __fmul_rn(nl[q], nx[q]));
+        for (int k = k0 + kSide; k < k1; ++k)
         {
             const int f = losort[k];
             sum = __fadd_rn(sum, __fmul_rn(lower[f], x[low[f]]));
         }
         y[i] = sum;
-        if (w) acc = (double)w[i] * (double)sum;
+        if (w) acc = (double)wi * (double)sum;
     }
     if (!dot) return;
     const double part = block_sum(acc, sh);
-    unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch + kTicketSlot);
     if (threadIdx.x == 0)
     {
         scratch[blockIdx.x] = part;
@@ -220,17 +274,17 @@ extern "C" int cf_ldu_spmv_dot_noalloc(int32_t nCells, const float* diag, const 
     double* scratch = nullptr;
     int rc = scratch_for_current_context(s, &scratch);
     if (rc != CF_OK) return rc;
-    if (dot)
-    {
-        // the counter must start at zero; the array keeps the last call's
-        // contents otherwise
-        cudaError_t e = cudaMemsetAsync(scratch + kTicketSlot, 0, sizeof(unsigned int), s);
-        if (e != cudaSuccess)
-            return cf::fail(CF_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-    }
+    // the completion counter of this call: zero when the library is loaded,
+    // set back to zero by the call's last block.  Calls take turns through the
+    // line's counters, so one whose kernel never ran to its end, or two that
+    // overlap against the contract, do not leave the next call a counter that
+    // is off (a cudaMemsetAsync before every launch did that for 2-3 us)
+    static std::atomic<unsigned int> turn{0};
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch + kTicketSlot) +
+                           turn.fetch_add(1, std::memory_order_relaxed) % kTickets;
     k_ldu_spmv_dot_noalloc<<<(unsigned)groups, kBlock, 0, s>>>(
         nCells, diag, upper, lower, lowAddr, uppAddr, ownStartAddr, losortAddr, losortStartAddr, x,
-        w, y, dot, scratch);
+        w, y, dot, scratch, ticket);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cf::fail(CF_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));

@@ -100,3 +100,42 @@ def test_noalloc_rejects_sizes_beyond_scratch(require_gpu):
     rc = L.cf_ldu_spmv_dot_noalloc(16_777_216 + 1, p, p, None, ip, ip, ip, ip, ip, p, p, p, None,
                                    None)
     assert rc == 9 and b"exceeds" in L.cf_last_error()
+
+
+def test_noalloc_many_faces_and_repeated_calls(require_gpu):
+    """Cells with none, four, five and many faces on either side (the loads
+    are batched by four), compared with a row-by-row FP32 sum in the call's
+    order, and more calls in a row than the library has completion counters."""
+    import torch
+
+    from metal4foam_b200 import _lib, mesh
+    n = 700
+    rng = np.random.default_rng(9)
+    pairs = {(0, j) for j in range(1, 60)} | {(j, n - 1) for j in range(600, n - 1)}
+    for width in (4, 5):
+        pairs |= {(i, i + d) for i in range(100, 300, 7) for d in range(1, width + 1)}
+    key = np.array(sorted(pairs), np.int64)
+    addr = mesh.ldu_addressing(n, key[:, 0].astype(np.int32), key[:, 1].astype(np.int32))
+    diag, x, w = (rng.standard_normal(n).astype(np.float32) for _ in range(3))
+    upper, lower = (rng.standard_normal(addr.nf).astype(np.float32) for _ in range(2))
+    y = diag * x
+    for i in range(n):
+        for f in range(addr.ownerStartAddr[i], addr.ownerStartAddr[i + 1]):
+            y[i] = np.float32(y[i] + upper[f] * x[addr.upperAddr[f]])
+        for k in range(addr.losortStartAddr[i], addr.losortStartAddr[i + 1]):
+            f = addr.losortAddr[k]
+            y[i] = np.float32(y[i] + lower[f] * x[addr.lowerAddr[f]])
+    dev = [torch.from_numpy(np.ascontiguousarray(v)).cuda()
+           for v in (diag, upper, lower, *addr.arrays(), x, w)]
+    d_y = torch.empty(n, dtype=torch.float32, device="cuda")
+    dots = torch.zeros(200, dtype=torch.float64, device="cuda")
+    L = _lib.load()
+    for k in range(200):
+        _lib.check(L.cf_ldu_spmv_dot_noalloc(n, *(_lib.ptr(t) for t in dev), _lib.ptr(d_y),
+                                             _lib.vp(dots.data_ptr() + 8 * k),
+                                             _lib.vp(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    assert np.array_equal(d_y.cpu().numpy(), y)
+    ref = float(w.astype(np.float64) @ y.astype(np.float64))
+    # (n terms of magnitude |w y| summed in FP64)
+    assert np.abs(dots.cpu().numpy() - ref).max() <= 1e-13 * np.abs(w * y).sum()
