@@ -122,8 +122,9 @@ typedef struct
                                   on, too while they fit one cluster, and up
                                   to what the SMs hold (about 900,000 cells)
                                   as one cooperative launch with the mesh
-                                  split over the SMs.  < 0: the graph loop
-                                  always                                   */
+                                  split over the SMs; the split is made by
+                                  the third solve on a topology.  < 0: the
+                                  graph loop always                        */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric
                                   V-cycle over aggregation levels (Galerkin

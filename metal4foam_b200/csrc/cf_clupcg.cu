@@ -568,8 +568,6 @@ void clu_release(cf_context* c)
     clu_plan_free(static_cast<CluPlan*>(c->clu));
     c->clu = nullptr;
     c->cluTried = false;
-    c->hostCol.clear();
-    c->hostSliceOff.clear();
 }
 
 int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int ips, int order,
@@ -581,12 +579,7 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
     {
         c->cluTried = true;
         if (c->hostSliceOff.empty()) return CF_OK;
-        HostLayout L;
-        L.col.swap(c->hostCol);
-        L.sliceOff.swap(c->hostSliceOff);
-        L.nslices = c->nslices;
-        L.nnzp = c->nnzp;
-        L.maxw = c->maxRowLen;
+        const HostLayout L = host_layout(c);
         CluPlan* plan = nullptr;
         const int ctas = std::min(CLU_MAX_CTAS, (c->n + CLU_T - 1) / CLU_T);
         if (clu_plan_build(c->n, L, !c->identityPerm, ctas, 0, 0, c->stream, &plan) != CF_OK)

@@ -90,6 +90,9 @@ void free_topology(cf_context* c)
     amg_release(c);
     resident_release(c);
     clu_release(c);
+    c->solves = 0;
+    c->hostCol.clear();
+    c->hostSliceOff.clear();
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
     c->graphs.clear();
     for (void* p : c->topoAllocs) cudaFree(p);
@@ -243,6 +246,17 @@ int check_addressing(int32_t n, int32_t nf, const int32_t* low, const int32_t* u
                      const int32_t* own, const int32_t* los, const int32_t* losS)
 {
     return validate_addressing(n, nf, low, upp, own, los, losS);
+}
+
+HostLayout host_layout(const cf_context* c)
+{
+    HostLayout L;
+    L.col = c->hostCol;
+    L.sliceOff = c->hostSliceOff;
+    L.nslices = c->nslices;
+    L.nnzp = c->nnzp;
+    L.maxw = c->maxRowLen;
+    return L;
 }
 
 // Internal ordering + SELL-32 layout of one mesh on the host.
@@ -725,8 +739,7 @@ extern "C" int cf_set_topology(cf_context* c, int32_t n, int32_t nf, const int32
     CF_CUDA(cudaMemsetAsync(c->d_D, 0, sizeof(float) * 3 * N, c->stream));
     CF_CUDA(cudaMemsetAsync(c->d_r64, 0, sizeof(double) * N, c->stream));
     CF_CUDA(cudaStreamSynchronize(c->stream));
-    CF_TRY(resident_build(c, L));
-    if (n <= CLU_MAX_ROWS && maxw <= 6)
+    if (n <= RESIDENT_MAX_ROWS && maxw <= 6)
     {
         c->hostCol.swap(col);
         c->hostSliceOff.swap(sliceOff);

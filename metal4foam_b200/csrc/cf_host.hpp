@@ -120,7 +120,9 @@ struct cf_context
     void* resident = nullptr;              // split of the mesh for resident inner solves (cf_resident.cu)
     void* clu = nullptr;                   // split of a small mesh over one cluster (cf_clupcg.cu)
     bool cluTried = false;                 // the split has been made, or cannot be
-    std::vector<int32_t> hostCol;          // host copy of the columns, kept for that split
+    bool residentTried = false;
+    int solves = 0;                        // cudaPCG solves on this topology so far
+    std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
     bool amgActive = false;                // inner PCG iterations use the V-cycle
     int clusterShift = 10;                 // log2(rows per CTA) of the cluster PCG for this mesh
@@ -261,19 +263,24 @@ void clu_release(cf_context* c);
 // log2(rows per CTA) of the cluster PCG for an n-row mesh: the smallest
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);
+// The host layout a split needs, from the copies the context keeps.
+HostLayout host_layout(const cf_context* c);
 int persistent_status(cf_context* c);
 
-// Inner PCG as one launch with the mesh split over the SMs (cf_resident.cu).
-// Meshes of at least RESIDENT_MIN_ROWS_PER_SM rows per SM get a split with
-// their topology; resident_inner runs and completes one inner solve (state
-// in h_st and d_st, the returned correction in d_D) when the context has
-// one and no other resident launch of the process runs on the device; *ran
-// tells whether it did.
+// Inner PCG as one launch with the mesh split over the SMs (cf_resident.cu),
+// for meshes of at least RESIDENT_MIN_ROWS_PER_SM rows per SM that fit.  The
+// split is made once per topology, by its RESIDENT_AFTER_SOLVES + 1st solve:
+// it takes the host as long as 5 to 10 solves save (25 ms at 300K cells), so a
+// mesh that is solved on once or twice does without.  resident_inner runs and
+// completes one inner solve (state in h_st and d_st, the returned correction
+// in d_D) when there is a split and no other resident launch of the process
+// runs on the device; *ran tells whether it did.
 constexpr int RESIDENT_MIN_ROWS_PER_SM = 128;
+constexpr int RESIDENT_AFTER_SOLVES = 2;
+constexpr int RESIDENT_MAX_ROWS = 1 << 20;   // no device holds more on its SMs
 struct InnerRun;
 InnerRun inner_run(const cf_context* c, const double* mean, double target, int maxIter, int ips,
                    int order, int stagLimit);
-int resident_build(cf_context* c, const HostLayout& L);
 void resident_release(cf_context* c);
 int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,
                    int order, int stagLimit, bool* ran);

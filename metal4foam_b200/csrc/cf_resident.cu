@@ -840,26 +840,38 @@ void resident_release(cf_context* c)
 {
     res_plan_free(static_cast<ResPlan*>(c->resident));
     c->resident = nullptr;
+    c->residentTried = false;
 }
 
-int resident_build(cf_context* c, const HostLayout& L)
+namespace {
+
+void resident_build(cf_context* c)
 {
-    resident_release(c);
     const int nparts = std::min(c->numSMs, RES_MAX_PARTS);
-    if (!c->coopLaunch || c->n < RESIDENT_MIN_ROWS_PER_SM * nparts || L.maxw < 4) return CF_OK;
+    if (!c->coopLaunch || c->n > (long long)nparts * RES_MAX_ROWS || c->hostSliceOff.empty()) return;
     ResPlan* p = nullptr;
-    if (res_plan_build(c->device, c->n, L, !c->identityPerm, nparts, 0, 0, c->stream, &p) != CF_OK)
+    if (res_plan_build(c->device, c->n, host_layout(c), !c->identityPerm, nparts, 0, 0, c->stream,
+                       &p) != CF_OK)
         cudaGetLastError();   // no memory for the split: the graph path
     c->resident = p;
-    return CF_OK;
 }
+
+}  // namespace
 
 int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,
                    int order, int stagLimit, bool* ran)
 {
     *ran = false;
+    if (maxIter <= 0 || c->solves < RESIDENT_AFTER_SOLVES ||
+        c->n < RESIDENT_MIN_ROWS_PER_SM * c->numSMs || c->maxRowLen < 4)
+        return CF_OK;
+    if (!c->residentTried)
+    {
+        c->residentTried = true;
+        resident_build(c);
+    }
     const ResPlan* p = static_cast<const ResPlan*>(c->resident);
-    if (!p || maxIter <= 0) return CF_OK;
+    if (!p) return CF_OK;
     // (another resident launch on the device: the graph path)
     std::unique_lock<std::mutex> turn(res_device_lock(c->device), std::try_to_lock);
     if (!turn.owns_lock()) return CF_OK;

@@ -249,9 +249,11 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
         bool resident = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
         // in one cluster up to 16,384 rows when their columns lie mostly in
-        // their own CTA (as the other cluster form) and from where the split
-        // over all SMs starts
-        if (c->n <= 16384 ? c->clusterRemote <= 0.25 : c->resident && c->n <= CLU_MAX_ROWS)
+        // their own CTA (as the other cluster form) and where the split over
+        // all SMs would start
+        if (c->n <= 16384 ? c->clusterRemote <= 0.25
+                          : c->n <= CLU_MAX_ROWS && c->solves >= RESIDENT_AFTER_SOLVES &&
+                                c->n >= RESIDENT_MIN_ROWS_PER_SM * c->numSMs && c->maxRowLen >= 4)
             CF_TRY(clu_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
         if (!resident)
             CF_TRY(resident_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
@@ -547,6 +549,7 @@ int solve_device(cf_context* c, int solver, double* psi_dev, const double* src_d
         perf->nRestarts = outer;
         perf->singular = singular;
     }
+    if (!bicg && !gamg && perf->solved) ++c->solves;
     perf->converged =
         check_convergence(o->tolerance, o->relTol, perf->initialResidual, perf->finalResidual);
     k_l2<<<grid_for(c, (const void*)k_l2, n), NT, 0, s>>>(n, c->d_r64, c->d_b, c->d_drv,
@@ -606,8 +609,10 @@ extern "C" int cf_pcg(cf_context* c, const double* r, double targetResSum, int32
                                 cudaMemcpyHostToDevice, c->stream));
     }
     CF_TRY(upload_r64(c, r));
-    return inner_solve(c, 0, nullptr, targetResSum, maxIter, iterationsPerSync,
-                       chebOrder > 1 ? chebOrder : 1, 1, stats);
+    CF_TRY(inner_solve(c, 0, nullptr, targetResSum, maxIter, iterationsPerSync,
+                       chebOrder > 1 ? chebOrder : 1, 1, stats));
+    ++c->solves;
+    return CF_OK;
 }
 
 extern "C" int cf_bicgstab(cf_context* c, const double* r, double targetResSum, int32_t maxIter,
