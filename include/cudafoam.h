@@ -113,7 +113,7 @@ typedef struct
                                   are at most this many, the inner loop of
                                   every system runs as one cooperative
                                   launch per restart; 0 (default): never   */
-    int32_t clusterMaxCells;   /* cudaPCG with graph = 1.  0 (default): meshes
+    int32_t clusterMaxCells;   /* with graph = 1.  0 (default): cudaPCG meshes
                                   of at most 16384 cells whose columns lie
                                   mostly in their own CTA run each inner
                                   solve inside one thread-block cluster of
@@ -123,8 +123,10 @@ typedef struct
                                   to what the SMs hold (about 900,000 cells)
                                   as one cooperative launch with the mesh
                                   split over the SMs; the split is made by
-                                  the third solve on a topology.  < 0: the
-                                  graph loop always                        */
+                                  the third solve on a topology.
+                                  cudaPBiCGStab: meshes of up to 40960 cells
+                                  with at most 6 neighbours per cell in one
+                                  cluster.  < 0: the graph loop always     */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric
                                   V-cycle over aggregation levels (Galerkin

@@ -429,16 +429,37 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long
         (long long)n * std::max(4, (int)L.maxw) > CLU_MAX_ENTRIES)
         return CF_OK;
     ResHost H;
+    try
+    {
+        if (!res_partition(n, L, ordered, ctas, H, 4)) return CF_OK;
+    }
+    catch (...)
+    {
+        return CF_OK;   // no memory for the split
+    }
+    int rows = 1;
+    for (int R : {1, 2, 3, 4, 6, 8, 10})
+    {
+        rows = R;
+        if (H.maxLocP <= R * CLU_T) break;
+    }
+    const int threads = ((H.maxLocP + rows - 1) / rows + 31) / 32 * 32;
+    return clu_plan_upload(H, ctas, 3, 3, entOff, rowOff, kernel_of(H.W, rows), rows, threads, s,
+                           plan);
+}
+
+int clu_plan_upload(ResHost& H, int ctas, int buffers, int nd, long long entOff, int rowOff,
+                    const void* fn, int R, int threads, cudaStream_t s, CluPlan** plan)
+{
+    *plan = nullptr;
+    const int W = H.W;
+    const int halo = std::max(H.maxHalo, 1);
     std::vector<unsigned int> dest;
     CluPlan* p = nullptr;
     int ndest = 0;
-    int halo = 0;
-    const int W = std::max(4, (int)L.maxw);
     try
     {
-        if (!res_partition(n, L, ordered, ctas, H, W)) return CF_OK;
-        halo = std::max(H.maxHalo, 1);
-        // readers of every boundary row
+        // readers of every row that has some
         std::vector<int> slotRow(H.slots), count(H.slots, 0);
         for (const ResPart& q : H.parts)
             for (int l = 0; l < q.nb; ++l) slotRow[q.llBase + l] = q.rowBase + l;
@@ -474,14 +495,10 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long
         return CF_OK;   // no memory for the split
     }
     p->W = W;
-    p->R = 1;
-    for (int R : {1, 2, 3, 4, 6, 8, 10})
-    {
-        p->R = R;
-        if (H.maxLocP <= R * CLU_T) break;
-    }
-    p->threads = ((H.maxLocP + p->R - 1) / p->R + 31) / 32 * 32;
-    p->smem = sizeof(float) * 3 * (size_t)(H.maxLocP + 2 * halo + 2);
+    p->R = R;
+    p->fn = fn;
+    p->threads = threads;
+    p->smem = sizeof(float) * buffers * (size_t)(H.maxLocP + 2 * halo + 2);
     p->split.rowsP = H.rowsP;
     p->split.ndest = ndest;
     p->split.ctas = ctas;
@@ -489,7 +506,6 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long
     p->split.halo = halo;
     // the attributes are the function's, shared by every context of the
     // process: one value, so no solve lowers it under another's launch
-    const void* fn = kernel_of(W, p->R);
     int clusters = 0;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
@@ -523,7 +539,7 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long
     const size_t dwAt = (k.host.size() + 255) & ~(size_t)255;
     char* base = nullptr;
     int rc = CF_OK;
-    if (cudaMalloc((void**)&base, dwAt + sizeof(float) * 3 * (size_t)H.rowsP) != cudaSuccess)
+    if (cudaMalloc((void**)&base, dwAt + sizeof(float) * nd * (size_t)H.rowsP) != cudaSuccess)
         rc = fail(CF_ERR_CUDA, "cluster split: cudaMalloc");
     if (rc == CF_OK) p->allocs.push_back(base);
     if (rc == CF_OK &&
@@ -546,6 +562,18 @@ int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long
     return CF_OK;
 }
 
+int clu_launch_fn(const void* fn, int ctas, int threads, size_t smem, void** args, int count,
+                  cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    config(ctas, threads, smem, count, s, &cfg, &attr);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+    if (e != cudaSuccess)
+        return fail(CF_ERR_CUDA, std::string("cluster launch: ") + cudaGetErrorString(e));
+    return CF_OK;
+}
+
 int clu_launch(int W, int R, int ctas, int threads, size_t smem, const CluSys* one,
                const CluSys* d_list, int count, cudaStream_t s)
 {
@@ -553,14 +581,8 @@ int clu_launch(int W, int R, int ctas, int threads, size_t smem, const CluSys* o
     a.list = d_list;
     if (one) a.one = *one;
     else std::memset((void*)&a.one, 0, sizeof(a.one));
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    config(ctas, threads, smem, count, s, &cfg, &attr);
     void* args[] = {(void*)&a};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel_of(W, R), args);
-    if (e != cudaSuccess)
-        return fail(CF_ERR_CUDA, std::string("cluster launch: ") + cudaGetErrorString(e));
-    return CF_OK;
+    return clu_launch_fn(kernel_of(W, R), ctas, threads, smem, args, count, s);
 }
 
 void clu_release(cf_context* c)

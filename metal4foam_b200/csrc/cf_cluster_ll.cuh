@@ -47,6 +47,7 @@ struct CluPlan
 {
     int W = 0, R = 0, threads = 0;
     size_t smem = 0;
+    const void* fn = nullptr;
     CluSplit split = {};
     float* dw = nullptr;
     std::vector<void*> allocs;
@@ -59,6 +60,13 @@ struct HostLayout;
 int clu_plan_build(int n, const HostLayout& L, bool ordered, int ctas, long long entOff,
                    int rowOff, cudaStream_t s, CluPlan** plan);
 void clu_plan_free(CluPlan* plan);
+// Parts of the above for other cluster kernels: a split (of `ctas` parts) in
+// the common layout onto the device, with room for nd corrections, for a
+// kernel that keeps `buffers` gathered vectors in shared memory.
+int clu_plan_upload(ResHost& H, int ctas, int buffers, int nd, long long entOff, int rowOff,
+                    const void* fn, int R, int threads, cudaStream_t s, CluPlan** plan);
+int clu_launch_fn(const void* fn, int ctas, int threads, size_t smem, void** args, int count,
+                  cudaStream_t s);
 // One launch: the system `one`, or the `count` systems of d_list, whose plans
 // share W, R and the number of CTAs (threads, smem: the largest of theirs).
 int clu_launch(int W, int R, int ctas, int threads, size_t smem, const CluSys* one,

@@ -90,6 +90,7 @@ void free_topology(cf_context* c)
     amg_release(c);
     resident_release(c);
     clu_release(c);
+    clu_bicg_release(c);
     c->solves = 0;
     c->hostCol.clear();
     c->hostSliceOff.clear();
@@ -902,6 +903,9 @@ int context_clone_sync(cf_context* src, cf_context* c)
     c->val32Sym = src->val32Sym;
     c->transposed = src->transposed;
     c->waitPolls = src->waitPolls;
+    c->cluBicg = src->cluBicg;   // (made before: clu_bicg_prepare)
+    c->cluBicgTried = true;
+    c->cluBicgShared = true;
     cf_spmv_config k;
     CF_TRY(cf_get_spmv_config(src, &k));
     return cf_set_spmv_config(c, &k);

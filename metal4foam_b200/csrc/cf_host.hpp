@@ -121,6 +121,9 @@ struct cf_context
     void* clu = nullptr;                   // split of a small mesh over one cluster (cf_clupcg.cu)
     bool cluTried = false;                 // the split has been made, or cannot be
     bool residentTried = false;
+    void* cluBicg = nullptr;               // the same for cudaPBiCGStab (cf_clubicg.cu)
+    bool cluBicgTried = false;
+    bool cluBicgShared = false;            // (a clone's: its source's)
     int solves = 0;                        // cudaPCG solves on this topology so far
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
@@ -260,6 +263,11 @@ constexpr int CLU_MAX_ROWS = 40960;
 int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int ips, int order,
               int stagLimit, bool* ran);
 void clu_release(cf_context* c);
+// The inner BiCGStab of a small mesh in one cluster (cf_clubicg.cu), the graph
+// loop's result bit for bit; _prepare makes the split (once per topology).
+void clu_bicg_prepare(cf_context* c);
+int clu_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagLimit, bool* ran);
+void clu_bicg_release(cf_context* c);
 // log2(rows per CTA) of the cluster PCG for an n-row mesh: the smallest
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);

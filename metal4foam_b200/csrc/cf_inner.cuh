@@ -61,7 +61,11 @@ __device__ __forceinline__ void inner_after_apply(InnerState& S, bool first, dou
 // without its error word, which another CTA may set at any time.
 __device__ __forceinline__ void inner_finish(InnerState& S, InnerState* st, bool store)
 {
-    if (S.bestRes < S.finalResSum)
+    if (S.early)   // BiCGStab's |s| exit returns its last iterate
+    {
+        S.sel = S.cur;
+    }
+    else if (S.bestRes < S.finalResSum)
     {
         S.sel = S.best;
         S.finalResSum = S.bestRes;

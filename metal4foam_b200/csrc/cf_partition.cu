@@ -376,4 +376,72 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
     return true;
 }
 
+// Consecutive ranges of rowsPerPart rows (whole slices), rows in the internal
+// order; the exchange slot of a row is the row itself.
+bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int width)
+{
+    const int W = std::max(width, (int)L.maxw);
+    if (W < 1 || W > 8 || rowsPerPart < SLICE || rowsPerPart % SLICE || n < 1) return false;
+    const int nparts = (n + rowsPerPart - 1) / rowsPerPart;
+    R.W = W;
+    R.rowsP = R.slots = nparts * rowsPerPart;
+    R.maxLocP = R.maxHalo = 0;
+    R.parts.assign(nparts, ResPart());
+    R.rowMap.assign((size_t)R.rowsP, -1);
+    for (int r = 0; r < n; ++r) R.rowMap[r] = r;
+    R.idx.resize((size_t)R.rowsP * W);
+    R.emap.assign((size_t)R.rowsP * W, -1);
+    R.haloSlot.clear();
+    std::vector<int32_t> h;
+    for (int p = 0; p < nparts; ++p)
+    {
+        ResPart& P = R.parts[p];
+        const int r0 = p * rowsPerPart;
+        P.rowBase = P.llBase = r0;
+        P.nloc = P.nb = std::min(rowsPerPart, n - r0);
+        P.nlocP = (P.nloc + SLICE - 1) / SLICE * SLICE;
+        auto each = [&](int r, auto fn) {
+            const int s = r / SLICE;
+            const int b0 = L.sliceOff[s];
+            const int w = (L.sliceOff[s + 1] - b0) / SLICE;
+            for (int j = 0; j < w; ++j)
+            {
+                const int32_t e = b0 + SLICE * j + r % SLICE;
+                if (L.col[e] != -1) fn(e, L.col[e] & 0x7fffffff);
+            }
+        };
+        h.clear();
+        for (int r = r0; r < r0 + P.nloc; ++r)
+            each(r, [&](int, int c) {
+                if (c < r0 || c >= r0 + P.nloc) h.push_back(c);
+            });
+        std::sort(h.begin(), h.end());
+        h.erase(std::unique(h.begin(), h.end()), h.end());
+        P.nh = (int)h.size();
+        P.haloBase = (int)R.haloSlot.size();
+        R.haloSlot.insert(R.haloSlot.end(), h.begin(), h.end());
+        R.maxLocP = std::max(R.maxLocP, P.nlocP);
+        R.maxHalo = std::max(R.maxHalo, P.nh);
+        if (P.nlocP + P.nh + 1 > 65535) return false;
+        for (int l = 0; l < P.nlocP; ++l)
+        {
+            const long long sb = ((long long)P.rowBase + l / SLICE * SLICE) * W;
+            int k = 0;
+            if (l < P.nloc)
+                each(r0 + l, [&](int e, int c) {
+                    const size_t at = (size_t)pair_index(sb, W, k, l % SLICE);
+                    R.idx[at] = (uint16_t)(c >= r0 && c < r0 + P.nloc
+                                               ? c - r0
+                                               : P.nlocP + (std::lower_bound(h.begin(), h.end(), c) -
+                                                            h.begin()));
+                    R.emap[at] = e;
+                    ++k;
+                });
+            for (; k < W; ++k)
+                R.idx[(size_t)pair_index(sb, W, k, l % SLICE)] = (uint16_t)(P.nlocP + P.nh);
+        }
+    }
+    return true;
+}
+
 }  // namespace cf

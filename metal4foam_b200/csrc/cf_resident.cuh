@@ -84,5 +84,8 @@ int res_reset(const ResPlan* plan, cudaStream_t s);
 // are wider than 8.  Rows are padded to `width` entries at least.
 bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R,
                    int width = 0);
+// The same with consecutive ranges of rowsPerPart rows (whole slices) in the
+// internal order; every row counts as read elsewhere.
+bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int width);
 
 }  // namespace cf

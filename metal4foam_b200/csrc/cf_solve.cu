@@ -242,7 +242,16 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
         c->lastInnerKind = kind;
         return CF_OK;
     };
-    // the whole inner solve as one launch on the mesh's split over the SMs
+    // the whole inner solve as one launch, in one cluster or on the mesh's
+    // split over the SMs
+    if (kind == 1 && useGraph && clusterMax >= 0 && spmv_default(c) && !mean)
+    {
+        bool whole = false;
+        CF_CUDA(cudaEventRecord(c->ev0, s));
+        CF_TRY(clu_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
+        c->pendingBodyKernels = 0;
+        if (whole) return finish();
+    }
     if (kind == 0 && useGraph && clusterMax >= 0 && persistMax <= 0 && spmv_default(c) &&
         !c->amgActive)
     {

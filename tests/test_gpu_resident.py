@@ -162,6 +162,67 @@ def test_cluster_equals_graph(require_gpu, name):
     ctx.close()
 
 
+# cudaPBiCGStab in one cluster: one 256-row block, its last row and a second
+# block, one block per CTA, two blocks per CTA, every number of blocks per
+# thread, the largest mesh and the first that is too large (launches as the
+# graph loop)
+BICG = {
+    "one_block": (lambda: mesh.upwind3d((16, 15), seed=1), {}),
+    "two_blocks": (lambda: mesh.upwind3d((257, 1, 1), seed=2), {}),
+    "sixteen_ctas": (lambda: mesh.upwind3d((64, 64), seed=3), dict(tolerance=1e-6)),
+    "nine_ctas": (lambda: mesh.upwind3d((17, 241, 1), seed=4), {}),
+    "three_blocks": (lambda: mesh.upwind3d((25, 23, 21), seed=5), {}),
+    "six_blocks": (lambda: mesh.upwind3d((30, 29, 25), seed=6), dict(iterationsPerSync=1)),
+    "max_iter": (lambda: mesh.upwind3d((25, 23, 21), seed=7), dict(maxIter=9, maxRestarts=2)),
+    "symmetric": (lambda: mesh.varcoeff3d((20, 18, 16), seed=8), {}),
+    "prism": (lambda: mesh.prism3d((24, 24, 16), seed=9), dict(tolerance=1e-6)),
+    "ten_blocks": (lambda: mesh.upwind3d((32, 32, 40), seed=10), dict(tolerance=1e-6)),
+    "too_large": (lambda: mesh.upwind3d((37, 36, 31), seed=11), dict(tolerance=1e-6)),
+}
+
+
+@pytest.mark.parametrize("name", BICG)
+def test_cluster_bicgstab_equals_graph(require_gpu, name):
+    """Every sum folds in the graph loop's order, so every field is equal."""
+    make, kw = BICG[name]
+    s = make()
+    ctx = _lib.Context(0)
+    ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
+    ctx.set_coeffs(s.diag, s.upper, s.lower)
+
+    def run(cluster):
+        x = np.zeros(s.n)
+        l0 = ctx.kernel_launches()
+        opts = dict(tolerance=1e-8, maxIter=5000, clusterMaxCells=cluster)
+        opts.update(kw)
+        p = ctx.solve(_lib.CF_SOLVER_PBICGSTAB, x, s.source, _lib.default_options(**opts))
+        return x, p, ctx.kernel_launches() - l0
+
+    xg, pg, lg = run(-1)
+    for _ in range(2):
+        xr, pr, lr = run(0)
+        assert (lr == lg) if name == "too_large" else (lr < lg), (lr, lg)
+        for f in FIELDS + ("finalResSum32",):
+            assert getattr(pr, f) == getattr(pg, f), (f, getattr(pr, f), getattr(pg, f))
+        assert np.array_equal(xr, xg)
+    ctx.set_wait_limit(1)
+    x1, p1, _ = run(0)
+    assert np.array_equal(x1, xg) and p1.nIterations == pg.nIterations
+    ctx.set_wait_limit(0)
+    # three components, each in a cluster of its own on the shared split
+    rng = np.random.default_rng(12)
+    b = rng.standard_normal((3, s.n))
+    opts = _lib.default_options(tolerance=1e-7, maxIter=5000)
+    psi = np.zeros((3, s.n))
+    perfs = ctx.solve_multi(_lib.CF_SOLVER_PBICGSTAB, psi, b, opts)
+    for k in range(3):
+        x = np.zeros(s.n)
+        p = ctx.solve(_lib.CF_SOLVER_PBICGSTAB, x, b[k],
+                      _lib.default_options(tolerance=1e-7, maxIter=5000, clusterMaxCells=-1))
+        assert np.array_equal(psi[k], x) and p.nIterations == perfs[k].nIterations
+    ctx.close()
+
+
 def test_resident_size_limits(require_gpu):
     """Just below the first size and just above the last: the graph loop
     (same launches with and without)."""
