@@ -126,7 +126,9 @@ typedef struct
                                   the third solve on a topology.
                                   cudaPBiCGStab: meshes of up to 40960 cells
                                   with at most 6 neighbours per cell in one
-                                  cluster.  < 0: the graph loop always     */
+                                  cluster, larger ones up to 6144 cells per
+                                  SM (about 900,000) as one cooperative
+                                  launch.  < 0: the graph loop always      */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric
                                   V-cycle over aggregation levels (Galerkin

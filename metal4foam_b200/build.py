@@ -16,7 +16,7 @@ SOURCES = ["cf_context.cu", "cf_solve.cu", "cf_batched.cu", "cf_adjoint.cu", "cf
            "cf_multi.cu", "cf_tune.cu",
            "cf_persist.cu", "cf_cluster.cu", "cf_amg.cu", "cf_many.cu", "cf_check.cu",
            "cf_coupled.cu", "cf_partition.cu", "cf_resident.cu", "cf_clupcg.cu",
-           "cf_clubicg.cu"]
+           "cf_clubicg.cu", "cf_resbicg.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 

@@ -91,6 +91,7 @@ void free_topology(cf_context* c)
     resident_release(c);
     clu_release(c);
     clu_bicg_release(c);
+    res_bicg_release(c);
     c->solves = 0;
     c->hostCol.clear();
     c->hostSliceOff.clear();
@@ -906,6 +907,7 @@ int context_clone_sync(cf_context* src, cf_context* c)
     c->cluBicg = src->cluBicg;   // (made before: clu_bicg_prepare)
     c->cluBicgTried = true;
     c->cluBicgShared = true;
+    c->waitTurn = true;          // (components take turns on the device)
     cf_spmv_config k;
     CF_TRY(cf_get_spmv_config(src, &k));
     return cf_set_spmv_config(c, &k);

@@ -124,6 +124,9 @@ struct cf_context
     void* cluBicg = nullptr;               // the same for cudaPBiCGStab (cf_clubicg.cu)
     bool cluBicgTried = false;
     bool cluBicgShared = false;            // (a clone's: its source's)
+    void* resBicg = nullptr;               // words of resident BiCGStab launches (cf_resbicg.cu)
+    bool resBicgTried = false;
+    bool waitTurn = false;                 // waits for a resident launch on the device to end
     int solves = 0;                        // cudaPCG solves on this topology so far
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
@@ -268,6 +271,9 @@ void clu_release(cf_context* c);
 void clu_bicg_prepare(cf_context* c);
 int clu_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagLimit, bool* ran);
 void clu_bicg_release(cf_context* c);
+// The same for larger meshes as one cooperative launch (cf_resbicg.cu).
+int res_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagLimit, bool* ran);
+void res_bicg_release(cf_context* c);
 // log2(rows per CTA) of the cluster PCG for an n-row mesh: the smallest
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);

@@ -164,8 +164,7 @@ def test_cluster_equals_graph(require_gpu, name):
 
 # cudaPBiCGStab in one cluster: one 256-row block, its last row and a second
 # block, one block per CTA, two blocks per CTA, every number of blocks per
-# thread, the largest mesh and the first that is too large (launches as the
-# graph loop)
+# thread, the largest mesh
 BICG = {
     "one_block": (lambda: mesh.upwind3d((16, 15), seed=1), {}),
     "two_blocks": (lambda: mesh.upwind3d((257, 1, 1), seed=2), {}),
@@ -177,15 +176,48 @@ BICG = {
     "symmetric": (lambda: mesh.varcoeff3d((20, 18, 16), seed=8), {}),
     "prism": (lambda: mesh.prism3d((24, 24, 16), seed=9), dict(tolerance=1e-6)),
     "ten_blocks": (lambda: mesh.upwind3d((32, 32, 40), seed=10), dict(tolerance=1e-6)),
-    "too_large": (lambda: mesh.upwind3d((37, 36, 31), seed=11), dict(tolerance=1e-6)),
 }
 
 
-@pytest.mark.parametrize("name", BICG)
-def test_cluster_bicgstab_equals_graph(require_gpu, name):
+def one_cell_more(s):
+    """s with a cell hung on its last one."""
+    low, upp = (np.append(a, v).astype(np.int32) for a, v in zip(s.addr.arrays()[:2], (s.n - 1, s.n)))
+    addr = mesh.ldu_addressing(s.n + 1, low, upp)
+    return mesh.LduSystem("more", addr, np.append(s.diag, 2.0), np.append(s.upper, -0.5),
+                          np.append(s.lower, -1.0), np.append(s.source, 1.0), np.zeros(s.n + 1))
+
+
+# one CTA per SM (1 m groups of 256 rows fill the m SMs once): the first
+# mesh too large for the cluster, a group of one row, the last and the first
+# number of groups before the blocks of each sum wrap (5, 6 and 8 per SM) for
+# each row width, numbers of groups per CTA that no kernel has, the largest
+# mesh and the first too large (launches as the graph loop)
+BICG_SMS = {
+    "first": (lambda m: mesh.upwind3d((37, 36, 31), seed=11), {}),
+    "one_row_more_2d": (lambda m: one_cell_more(mesh.upwind3d((2 * m, 256), seed=12)),
+                        dict(maxIter=40)),
+    "prism_5": (lambda m: mesh.prism3d((m // 2, 32, 64), seed=13), dict(maxIter=60)),
+    "prism_7": (lambda m: mesh.prism3d((m // 2, 52, 64), seed=14), dict(maxIter=60)),
+    "ab_full_3d": (lambda m: mesh.upwind3d((m, 32, 48), seed=15), {}),
+    "ab_wraps_3d": (lambda m: mesh.upwind3d((m, 32, 49), seed=16), dict(iterationsPerSync=3)),
+    "cd_full_2d": (lambda m: mesh.upwind3d((m, 1280), seed=17), dict(maxIter=60)),
+    "cd_wraps_2d": (lambda m: mesh.upwind3d((m, 1291), seed=18), dict(maxIter=60)),
+    "e_wraps_2d": (lambda m: mesh.upwind3d((m, 2051), seed=19), dict(maxIter=40)),
+    "symmetric_9": (lambda m: mesh.varcoeff3d((m, 45, 50), seed=20), dict(maxIter=50)),
+    "last": (lambda m: mesh.upwind3d((m, 64, 96), seed=21), dict(maxIter=30)),
+    "too_large": (lambda m: mesh.upwind3d((m, 64, 97), seed=22), dict(maxIter=30)),
+}
+
+
+@pytest.mark.parametrize("name", [*BICG, *BICG_SMS])
+def test_bicgstab_equals_graph(require_gpu, name):
     """Every sum folds in the graph loop's order, so every field is equal."""
-    make, kw = BICG[name]
-    s = make()
+    if name in BICG:
+        make, kw = BICG[name]
+        s = make()
+    else:
+        make, kw = BICG_SMS[name]
+        s = make(sms())
     ctx = _lib.Context(0)
     ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
     ctx.set_coeffs(s.diag, s.upper, s.lower)
@@ -209,16 +241,18 @@ def test_cluster_bicgstab_equals_graph(require_gpu, name):
     x1, p1, _ = run(0)
     assert np.array_equal(x1, xg) and p1.nIterations == pg.nIterations
     ctx.set_wait_limit(0)
-    # three components, each in a cluster of its own on the shared split
+    # three components, each in a cluster of its own on the shared split or in
+    # turn on all SMs
     rng = np.random.default_rng(12)
     b = rng.standard_normal((3, s.n))
-    opts = _lib.default_options(tolerance=1e-7, maxIter=5000)
+    limit = kw.get("maxIter", 5000)
+    opts = _lib.default_options(tolerance=1e-7, maxIter=limit)
     psi = np.zeros((3, s.n))
     perfs = ctx.solve_multi(_lib.CF_SOLVER_PBICGSTAB, psi, b, opts)
     for k in range(3):
         x = np.zeros(s.n)
         p = ctx.solve(_lib.CF_SOLVER_PBICGSTAB, x, b[k],
-                      _lib.default_options(tolerance=1e-7, maxIter=5000, clusterMaxCells=-1))
+                      _lib.default_options(tolerance=1e-7, maxIter=limit, clusterMaxCells=-1))
         assert np.array_equal(psi[k], x) and p.nIterations == perfs[k].nIterations
     ctx.close()
 
