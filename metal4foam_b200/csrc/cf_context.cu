@@ -907,7 +907,9 @@ int context_clone_sync(cf_context* src, cf_context* c)
     c->cluBicg = src->cluBicg;   // (made before: clu_bicg_prepare)
     c->cluBicgTried = true;
     c->cluBicgShared = true;
-    c->waitTurn = true;          // (components take turns on the device)
+    c->resBicg = src->resBicg;   // (res_bicg_prepare)
+    c->resBicgTried = true;
+    c->resBicgShared = true;
     cf_spmv_config k;
     CF_TRY(cf_get_spmv_config(src, &k));
     return cf_set_spmv_config(c, &k);

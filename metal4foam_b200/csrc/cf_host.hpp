@@ -16,6 +16,10 @@
 
 constexpr int CF_MAX_CHEB = 64;
 
+namespace cf {
+struct ResBicgTeam;
+}
+
 struct cf_context
 {
     // device / runtime (metalFoamBackend::Impl::init, metalFoamBackend.C:192-282)
@@ -124,9 +128,10 @@ struct cf_context
     void* cluBicg = nullptr;               // the same for cudaPBiCGStab (cf_clubicg.cu)
     bool cluBicgTried = false;
     bool cluBicgShared = false;            // (a clone's: its source's)
-    void* resBicg = nullptr;               // words of resident BiCGStab launches (cf_resbicg.cu)
+    void* resBicg = nullptr;               // plan of resident BiCGStab launches (cf_resbicg.cu)
     bool resBicgTried = false;
-    bool waitTurn = false;                 // waits for a resident launch on the device to end
+    bool resBicgShared = false;            // (a clone's: its source's)
+    cf::ResBicgTeam* resBicgTeam = nullptr; // clones that run their inner solves together
     int solves = 0;                        // cudaPCG solves on this topology so far
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
@@ -272,8 +277,14 @@ void clu_bicg_prepare(cf_context* c);
 int clu_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagLimit, bool* ran);
 void clu_bicg_release(cf_context* c);
 // The same for larger meshes as one cooperative launch (cf_resbicg.cu).
+void res_bicg_prepare(cf_context* c);
 int res_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagLimit, bool* ran);
 void res_bicg_release(cf_context* c);
+// Clones on host threads of their own whose inner solves run as one launch:
+// every member calls res_bicg_inner or leaves.  Null: each for itself.
+ResBicgTeam* res_bicg_team(cf_context* c, int members);
+void res_bicg_leave(ResBicgTeam* t);
+void res_bicg_team_free(ResBicgTeam* t);
 // log2(rows per CTA) of the cluster PCG for an n-row mesh: the smallest
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);

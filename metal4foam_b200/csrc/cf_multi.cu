@@ -1012,13 +1012,31 @@ int solve_multi_streams(cf_context* c, int32_t solver, int32_t nrhs, double* psi
     const int wantSym32 = c->hasLower ? 0 : 1;
     if (wantSym32 != c->val32Sym) CF_TRY(stage_vals(c, wantSym32));
     clu_bicg_prepare(c);   // (the clones share the split)
+    res_bicg_prepare(c);
     for (int w = 0; w < W; ++w) CF_TRY(context_clone_sync(c, c->clones[w]));
     // the clones' streams start after the work queued so far on this one
     CF_CUDA(cudaEventRecord(c->ev0, c->stream));
     for (int w = 0; w < W; ++w) CF_CUDA(cudaStreamWaitEvent(c->clones[w]->stream, c->ev0, 0));
     std::vector<int> rc(nrhs, CF_OK);
     std::vector<std::string> msg(nrhs);
-    auto run = [&](int w) {
+    // Meshes that run as one CTA per SM: up to three components in one launch
+    // (cf_resbicg.cu).
+    ResBicgTeam* const team = o->graph && o->clusterMaxCells >= 0 && nrhs == W
+                                  ? res_bicg_team(c, W) : nullptr;
+    if (W > 1 && !team)   // concurrent graph loops, which all SMs' CTAs would hold up
+        for (int w = 0; w < W; ++w) c->clones[w]->resBicg = nullptr;
+    auto run = [&](int w, ResBicgTeam* team) {
+        struct Member
+        {
+            cf_context* c;
+            ResBicgTeam* t;
+            ~Member()
+            {
+                c->resBicgTeam = nullptr;
+                if (t) res_bicg_leave(t);
+            }
+        } member{c->clones[w], team};
+        c->clones[w]->resBicgTeam = team;
         for (int k = w; k < nrhs; k += W)
         {
             double* p = psi + k * n;
@@ -1040,16 +1058,18 @@ int solve_multi_streams(cf_context* c, int32_t solver, int32_t nrhs, double* psi
     {
         try
         {
-            pool.emplace_back(run, w);
+            pool.emplace_back(run, w, team);
         }
         catch (...)
         {
             inlineRuns.push_back(w);   // no exception crosses the C ABI
+            if (team) res_bicg_leave(team);
         }
     }
-    run(0);
-    for (int w : inlineRuns) run(w);
+    run(0, team);
+    for (int w : inlineRuns) run(w, nullptr);
     for (auto& t : pool) t.join();
+    if (team) res_bicg_team_free(team);
     for (int k = 0; k < nrhs; ++k)
         if (rc[k] != CF_OK) return fail(rc[k], "component " + std::to_string(k) + ": " + msg[k]);
     for (int w = 0; w < W; ++w)

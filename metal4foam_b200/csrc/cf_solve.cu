@@ -249,9 +249,7 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
         bool whole = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
         CF_TRY(clu_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
-        // (smaller meshes that the cluster refuses: the graph loop)
-        if (!whole && c->n > NT * 160)
-            CF_TRY(res_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
+        if (!whole) CF_TRY(res_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
         c->pendingBodyKernels = 0;
         if (whole) return finish();
     }
