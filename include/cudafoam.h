@@ -128,7 +128,9 @@ typedef struct
                                   with at most 6 neighbours per cell in one
                                   cluster, larger ones up to 6144 cells per
                                   SM (about 900,000) as one cooperative
-                                  launch.  < 0: the graph loop always      */
+                                  launch.  GAMG: the levels of at most 4096
+                                  cells in one cluster.  < 0: the graph loop
+                                  always, launches for every level         */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric
                                   V-cycle over aggregation levels (Galerkin

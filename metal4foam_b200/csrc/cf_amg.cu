@@ -38,7 +38,8 @@
 // by the update kernel, its last post-smoothing step forms z.r and beta).
 // The restriction is formed by the kernel that starts the next level, and
 // the prolongation by the first post-smoothing step, which reads x + a P x'
-// on the fly, so a coarse level costs five launches.
+// on the fly, so a coarse level costs five launches.  The levels of at most
+// AMG_TAIL_ROWS cells run together in one cluster (ka_tail).
 #include "cudafoam.h"
 #include "cf_host.hpp"
 
@@ -50,9 +51,13 @@
 #include <string>
 #include <vector>
 
+#include <cooperative_groups.h>
+#include <cuda_pipeline.h>
+
 #include "cf_kernels.cuh"
 
 using namespace cf;
+namespace cg = cooperative_groups;
 
 #define AMG_CUDA(call)                                                          \
     do                                                                          \
@@ -86,6 +91,11 @@ constexpr int AMG_INV_THREADS = 1024;
 constexpr int AMG_MAX_AGG = 8;       // cells per root aggregate at most
 constexpr double AMG_STRONG = 0.08;  // strong coupling: |a_ij| >= this * sqrt(a_ii a_jj)
 constexpr int AMG_COARSE_DEGREE = 2; // smoother degree below level 0 (at most nSweeps)
+constexpr int AMG_TAIL_ROWS = 4096;  // levels up to here run in one cluster (ka_tail) ...
+constexpr int AMG_TAIL_CTAS = 8;     // ... of as many CTAs as lanes share a row
+constexpr int AMG_TAIL_T = 512;
+constexpr int AMG_TAIL_WHOLE = AMG_MAX_COARSEST;   // levels up to here: every CTA forms all rows
+constexpr int AMG_TAIL_SMEM = 220 * 1024;
 
 struct AmgLevel
 {
@@ -114,6 +124,14 @@ struct AmgLevel
     int* cfList = nullptr;
     int* intStart = nullptr;    // [nagg + 1] this level's faces inside each aggregate
     int* intList = nullptr;
+    // row-major copy of the operator for ka_tail: every row padded to tailW
+    // entries, tailM rows per CTA
+    int tailM = 0, tailW = 0;
+    float* tailVal = nullptr;
+    unsigned short* tailIdx = nullptr;   // 0xffff: no entry
+    int* tailMap = nullptr;              // SELL entry -> entry of the copy
+    int tailCtas = 0;                    // CTAs that share its rows (1: each has all)
+    std::vector<int> tailFine;           // first cell of the finer level of each CTA, and the end
     // host copies for cf_gamg_export: this level's faces (levels >= 1) and
     // the aggregate of each row (levels with a coarser one)
     std::vector<int> hLow, hUpp, hAgg;
@@ -124,6 +142,9 @@ struct AmgData
     int coarsestCap = 0;        // nCellsInCoarsestLevel the hierarchy was built for
     std::vector<AmgLevel> lv;
     std::vector<void*> allocs;
+    int tailFrom = 0;              // first level of the cluster (0: none)
+    int tailSmem = 0;
+    void* tailLevels = nullptr;    // TailLevel of every level from there on
     double* coarseInv = nullptr;   // [nc * nc] inverse of the coarsest operator (row-major)
     float* scale = nullptr;        // scaleCorrection of the current solve
     float hostScale = 1.0f;        // its host copy (source of the async upload)
@@ -286,13 +307,16 @@ __global__ void ka_coarse_diag(int nagg, const int* __restrict__ aggStart,
 
 // symmetric SELL values of a coarse level
 __global__ void ka_stage_vals(long long nnzp, const int* __restrict__ eface,
-                              const double* __restrict__ upper, float* __restrict__ val)
+                              const double* __restrict__ upper, float* __restrict__ val,
+                              const int* __restrict__ tailMap, float* __restrict__ tailVal)
 {
     for (long long e = (long long)blockIdx.x * NT + threadIdx.x; e < nnzp;
          e += (long long)gridDim.x * NT)
     {
         const int f = eface[e];
-        val[e] = f < 0 ? 0.0f : (float)upper[f];
+        const float v = f < 0 ? 0.0f : (float)upper[f];
+        val[e] = v;
+        if (tailMap) tailVal[tailMap[e]] = v;
     }
 }
 
@@ -304,9 +328,9 @@ __global__ void __launch_bounds__(AMG_INV_THREADS)
                      const int* __restrict__ eface, const double* __restrict__ upper,
                      const double* __restrict__ diag, int shift, double* __restrict__ inv)
 {
-    extern __shared__ double sm[];
-    double* M = sm;               // nc * nc
-    double* colp = sm + nc * nc;  // column p of the current step
+    extern __shared__ double sm64[];
+    double* M = sm64;               // nc * nc
+    double* colp = sm64 + nc * nc;  // column p of the current step
     const int t = threadIdx.x;
     const int nn = nc * nc;
     double dsum = 0.0;
@@ -559,6 +583,383 @@ __global__ void __launch_bounds__(NT) ka_step_lanes(DevSell A, const float* __re
 }
 
 
+// ------------------------------------------------------------------- tail
+
+// The V-cycle of the levels of at most AMG_TAIL_ROWS cells as one cluster of
+// eight CTAs.  On its own such a level costs five launches of about 3 us
+// whatever its size; here a phase costs a cluster barrier (0.35 us) and a
+// pass over shared memory, whose banks the gathers of wide rows keep busy: at
+// 1,138 and 179 cells 18 us in all, 4 of them to load the levels, at 2,720
+// cells about as much as the launches, so larger levels keep those.  Per
+// iteration 229 -> 213 us at 872K cells, 88 -> 74 at 30K, 376 -> 361 at
+// 128^3.  Every CTA holds tailM rows of each level's operator and all
+// of its iterates and residuals: the eight lanes that form a row together
+// store its new value to one CTA each.  (With the iterates in L2 the cluster was
+// no faster than the launches: a phase is two or three dependent trips.)
+// Per row the arithmetic is that of ka_restrict_init, ka_step_lanes<., 8, .>
+// and ka_restrict_coarse_solve.
+struct TailLevel
+{
+    int n, m, w;              // cells, rows per CTA, entries per row
+    int whole;                // every CTA has all rows
+    int fine[AMG_TAIL_CTAS + 1];   // first cell of the finer level of each CTA, and the end
+    const float* val;
+    const unsigned short* idx;
+    const float* diag;
+    const float* rD;
+    const int* aggStart;      // this level's cells as sets of the finer level's
+    const int* aggRows;
+    const int* agg;           // the coarser level's cell of each row
+    // byte offsets in shared memory
+    int oVal, oIdx, oDiag, oRD, oB, oW, oX0, oX1, oR, oAgg, oStart, oRows;
+};
+
+struct TailArgs
+{
+    const TailLevel* lv;            // finest first; the last is solved directly
+    int count, degree;
+    const float* rf;                // residual of the level above the finest
+    float* out;                     // the finest level's correction
+    const double* inv;
+    const float* scale;
+    const float* cc;
+    const InnerState* st;
+};
+
+// step j of a level (resid: the residual) from x, into `out` of every CTA, or
+// (global) into an array of all rows; cc: the polynomial, in shared memory
+__device__ __forceinline__ void tail_step(const TailLevel& L, char* sm, int rank, bool resid,
+                                       const float* x, float* out, float* global, const float* cc,
+                                       int j)
+{
+    const int lane = threadIdx.x & 31;
+    const int sub = lane & 7;
+    const float c2 = j > 0 ? cc[2 * j - 1] : 0.0f;
+    const float c3 = j > 0 ? cc[2 * j] : cc[0];
+    const float* val = reinterpret_cast<const float*>(sm + L.oVal);
+    const unsigned short* idx = reinterpret_cast<const unsigned short*>(sm + L.oIdx);
+    const float* diag = reinterpret_cast<const float*>(sm + L.oDiag);
+    const float* rD = reinterpret_cast<const float*>(sm + L.oRD);
+    const float* b = reinterpret_cast<const float*>(sm + L.oB);
+    float* w = reinterpret_cast<float*>(sm + L.oW);
+    const int first = L.whole ? 0 : rank * L.m;
+    float* to = L.whole ? out : cg::this_cluster().map_shared_rank(out, sub);
+    const int rows = min(L.m, L.n - first);
+    for (int i0 = (threadIdx.x >> 5) * 4; i0 < rows; i0 += AMG_TAIL_T / 8)
+    {
+        const int i = i0 + (lane >> 3);     // (m is a multiple of 4)
+        const bool valid = i < rows;
+        const float xr = valid ? x[first + i] : 0.0f;
+        const float bi = b[i];
+        const float di = diag[i];
+        const float wi = j > 0 ? w[i] : 0.0f;
+        const float ri = resid ? 0.0f : rD[i];
+        float off = 0.0f;
+        for (int k0 = sub; k0 < L.w; k0 += 32)
+        {
+            unsigned int c[4];
+            float v[4], y[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                c[q] = k0 + 8 * q < L.w ? idx[i * L.w + k0 + 8 * q] : 0xffffu;
+            if (c[0] == 0xffffu) break;     // (a row's entries come first)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+            {
+                v[q] = c[q] != 0xffffu ? val[i * L.w + k0 + 8 * q] : 0.0f;
+                y[q] = c[q] != 0xffffu ? x[c[q]] : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (c[q] != 0xffffu) off = __fadd_rn(off, __fmul_rn(v[q], y[q]));
+        }
+        __syncwarp();                       // (all lanes have read w)
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) off = __fadd_rn(off, __shfl_xor_sync(0xffffffffu, off, o));
+        const float v = __fadd_rn(__fmul_rn(di, xr), off);
+        float y;
+        if (resid)
+        {
+            y = __fsub_rn(bi, v);
+        }
+        else
+        {
+            const float s = __fmul_rn(__fmul_rn(c3, ri), __fsub_rn(bi, v));
+            const float wn = j > 0 ? __fadd_rn(__fmul_rn(c2, wi), s) : s;
+            if (sub == 0) w[i] = wn;
+            y = __fadd_rn(xr, wn);
+        }
+        if (!valid) continue;
+        if (global)
+        {
+            if (sub == 0 && (!L.whole || rank == 0)) global[first + i] = y;
+        }
+        else if (!L.whole || sub == 0)
+        {
+            to[first + i] = y;
+        }
+    }
+}
+
+// aggregate of local row i from the finer level's residual (the loads of a
+// few cells before their additions)
+__device__ __forceinline__ float tail_restrict(const TailLevel& L, const char* sm, int i,
+                                               const float* rf)
+{
+    const int* start = reinterpret_cast<const int*>(sm + L.oStart);
+    const int* rows = reinterpret_cast<const int*>(sm + L.oRows) - start[0];
+    const int q1 = start[i + 1];
+    float acc = 0.0f;
+    for (int q = start[i]; q < q1; q += 8)
+    {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = q + u < q1 ? rf[rows[q + u]] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (q + u < q1) acc = __fadd_rn(acc, v[u]);
+    }
+    return acc;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void tail_copy(char* to, const void* from, int count)
+{
+    for (int k = threadIdx.x; k < count; k += AMG_TAIL_T)
+        __pipeline_memcpy_async(to + (size_t)k * BYTES, static_cast<const char*>(from) + (size_t)k * BYTES,
+                                BYTES);
+}
+
+__global__ void __launch_bounds__(AMG_TAIL_T) ka_tail(const __grid_constant__ TailArgs a)
+{
+    extern __shared__ double sm64[];
+    char* sm = reinterpret_cast<char*>(sm64);
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const int tid = threadIdx.x;
+    const int last = a.count - 1;
+    const int done = a.st->done;
+    __shared__ TailLevel lv[AMG_MAX_LEVELS];
+    for (int k = tid; k < a.count * (int)(sizeof(TailLevel) / sizeof(int)); k += AMG_TAIL_T)
+        reinterpret_cast<int*>(lv)[k] = __ldg(reinterpret_cast<const int*>(a.lv) + k);
+    __shared__ float cc[2 * AMG_COARSE_DEGREE];
+    const float sc = __ldg(a.scale);
+    if (tid < 2 * a.degree - 1) cc[tid] = __ldg(a.cc + tid);
+    if (done) return;         // (the whole cluster)
+    __syncthreads();
+    const int nc = lv[last].n;
+    const int lane = tid & 31;
+    // this warp's row of the coarsest level's inverse
+    static_assert(AMG_TAIL_CTAS * AMG_TAIL_T / 32 >= AMG_MAX_COARSEST, "a row per warp");
+    const int ci = rank + AMG_TAIL_CTAS * (tid >> 5);
+    double inv[AMG_MAX_COARSEST / 32];
+#pragma unroll
+    for (int q = 0; q < AMG_MAX_COARSEST / 32; ++q)
+        inv[q] = ci < nc && lane + 32 * q < nc ? __ldg(a.inv + ci * nc + lane + 32 * q) : 0.0;
+    // everything the levels need, asked for at once
+    for (int l = 0; l <= last; ++l)
+    {
+        const TailLevel& L = lv[l];
+        const int at = L.whole ? 0 : rank;
+        const int r0 = min(L.n, at * L.m);
+        const int r1 = min(L.n, r0 + L.m);
+        tail_copy<4>(sm + L.oStart, L.aggStart + r0, r1 - r0 + 1);
+        tail_copy<4>(sm + L.oRows, L.aggRows + L.fine[at], L.fine[at + 1] - L.fine[at]);
+        if (l == last) break;
+        const size_t first = (size_t)at * L.m * L.w;
+        tail_copy<16>(sm + L.oVal, L.val + first, L.m * L.w / 4);
+        tail_copy<16>(sm + L.oIdx, L.idx + first, L.m * L.w / 8);
+        tail_copy<4>(sm + L.oDiag, L.diag + r0, r1 - r0);
+        tail_copy<4>(sm + L.oRD, L.rD + r0, r1 - r0);
+        tail_copy<4>(sm + L.oAgg, L.agg, L.n);
+    }
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    cl.sync();   // (also: every CTA runs before another stores to it)
+    const float c1 = cc[0];
+    const float* rf = a.rf;
+    auto sync = [&](const TailLevel& L) {
+        if (L.whole)
+            __syncthreads();
+        else
+            cl.sync();
+    };
+    for (int l = 0; l < last; ++l)
+    {
+        const TailLevel& L = lv[l];
+        float* xa = reinterpret_cast<float*>(sm + L.oX0);
+        float* xb = reinterpret_cast<float*>(sm + L.oX1);
+        float* r = reinterpret_cast<float*>(sm + L.oR);
+        const int first = L.whole ? 0 : rank * L.m;
+        for (int i = tid; i < L.m && first + i < L.n; i += AMG_TAIL_T)
+        {
+            const float acc = tail_restrict(L, sm, i, rf);
+            reinterpret_cast<float*>(sm + L.oB)[i] = acc;
+            const float v =
+                __fmul_rn(__fmul_rn(c1, reinterpret_cast<const float*>(sm + L.oRD)[i]), acc);
+            reinterpret_cast<float*>(sm + L.oW)[i] = v;
+            if (L.whole)
+            {
+                xa[i] = v;
+                continue;
+            }
+#pragma unroll
+            for (int k = 0; k < AMG_TAIL_CTAS; ++k) cl.map_shared_rank(xa, k)[first + i] = v;
+        }
+        sync(L);
+        for (int j = 1; j < a.degree; ++j)
+        {
+            tail_step(L, sm, rank, false, xa, xb, nullptr, cc, j);
+            sync(L);
+            float* t = xa;
+            xa = xb;
+            xb = t;
+        }
+        tail_step(L, sm, rank, true, xa, r, nullptr, cc, 0);
+        sync(L);
+        rf = r;
+    }
+    // the coarsest level: its right-hand side in every CTA, its rows shared
+    {
+        const TailLevel& L = lv[last];
+        float* b = reinterpret_cast<float*>(sm + L.oB);
+        float* x = reinterpret_cast<float*>(sm + L.oX0);
+        for (int k = tid; k < nc; k += AMG_TAIL_T) b[k] = tail_restrict(L, sm, k, rf);
+        __syncthreads();
+        if (ci < nc)
+        {
+            double acc = 0.0;
+#pragma unroll
+            for (int q = 0; q < AMG_MAX_COARSEST / 32; ++q)
+                if (lane + 32 * q < nc) acc += inv[q] * (double)b[lane + 32 * q];
+            acc = warp_sum(acc);
+            if (lane < AMG_TAIL_CTAS) cl.map_shared_rank(x, lane)[ci] = (float)acc;
+        }
+        cl.sync();
+    }
+    const float* xc = reinterpret_cast<const float*>(sm + lv[last].oX0);
+    for (int l = last - 1; l >= 0; --l)
+    {
+        const TailLevel& L = lv[l];
+        // (where degree - 1 steps have left the iterate)
+        float* xa = reinterpret_cast<float*>(sm + ((a.degree & 1) ? L.oX0 : L.oX1));
+        float* xb = reinterpret_cast<float*>(sm + ((a.degree & 1) ? L.oX1 : L.oX0));
+        const int* agg = reinterpret_cast<const int*>(sm + L.oAgg);
+        for (int k = tid; k < L.n; k += AMG_TAIL_T)
+            xa[k] = __fadd_rn(xa[k], __fmul_rn(sc, xc[agg[k]]));
+        __syncthreads();
+        for (int j = 0; j < a.degree; ++j)
+        {
+            const bool end = l == 0 && j + 1 == a.degree;
+            tail_step(L, sm, rank, false, xa, xb, end ? a.out : nullptr, cc, j);
+            if (!end) sync(L);
+            float* t = xa;
+            xa = xb;
+            xb = t;
+        }
+        xc = xa;
+    }
+}
+
+// Offsets of a tail that starts with level `from`; the shared memory it needs.
+int tail_layout(const AmgData* d, int from, TailLevel* lv)
+{
+    int at = 0;
+    auto take = [&](size_t bytes) {
+        const int o = at;
+        at += (int)((bytes + 15) / 16 * 16);
+        return o;
+    };
+    const int last = (int)d->lv.size() - 1;
+    for (int l = from; l <= last; ++l)
+    {
+        const AmgLevel& L = d->lv[l];
+        TailLevel T = {};
+        const size_t m = L.tailM;
+        T.n = L.n;
+        T.m = L.tailM;
+        T.w = L.tailW;
+        T.whole = L.tailCtas == 1;
+        int cells = 0;
+        for (int k = 0; k <= L.tailCtas; ++k)
+        {
+            T.fine[k] = L.tailFine[k];
+            if (k) cells = std::max(cells, T.fine[k] - T.fine[k - 1]);
+        }
+        T.oStart = take(sizeof(int) * (m + 1));
+        T.oRows = take(sizeof(int) * cells);
+        T.oB = take(sizeof(float) * m);
+        T.oX0 = take(sizeof(float) * L.n);
+        if (l < last)
+        {
+            T.oVal = take(sizeof(float) * m * L.tailW);
+            T.oIdx = take(sizeof(short) * m * L.tailW);
+            T.oDiag = take(sizeof(float) * m);
+            T.oRD = take(sizeof(float) * m);
+            T.oW = take(sizeof(float) * m);
+            T.oX1 = take(sizeof(float) * L.n);
+            T.oR = take(sizeof(float) * L.n);
+            T.oAgg = take(sizeof(int) * L.n);
+        }
+        if (lv) lv[l - from] = T;
+    }
+    return at;
+}
+
+// the finest level from which on everything fits (a single level below
+// stays with its one launch)
+int choose_tail(cf_context* c, AmgData* d)
+{
+    d->tailFrom = 0;
+    const int last = (int)d->lv.size() - 1;
+    for (int l = last - 1; l >= 1 && d->lv[l].tailM > 0; --l)
+    {
+        const int need = tail_layout(d, l, nullptr);
+        if (need > AMG_TAIL_SMEM) break;
+        d->tailFrom = l;
+        d->tailSmem = need;
+    }
+    int clusters = 0;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = AMG_TAIL_CTAS;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(AMG_TAIL_CTAS);
+    cfg.blockDim = dim3(AMG_TAIL_T);
+    cfg.dynamicSmemBytes = AMG_TAIL_SMEM;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (d->tailFrom &&
+        (cudaFuncSetAttribute(ka_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              AMG_TAIL_SMEM) != cudaSuccess ||
+         cudaOccupancyMaxActiveClusters(&clusters, ka_tail, &cfg) != cudaSuccess || clusters < 1))
+    {
+        cudaGetLastError();
+        d->tailFrom = 0;
+    }
+    if (!d->tailFrom) return CF_OK;
+    std::vector<TailLevel> lv(d->lv.size() - d->tailFrom);
+    tail_layout(d, d->tailFrom, lv.data());
+    for (size_t k = 0; k < lv.size(); ++k)
+    {
+        const AmgLevel& L = d->lv[d->tailFrom + k];
+        const AmgLevel& F = d->lv[d->tailFrom + k - 1];
+        lv[k].val = L.tailVal;
+        lv[k].idx = L.tailIdx;
+        lv[k].diag = L.diag32;
+        lv[k].rD = L.rD32;
+        lv[k].aggStart = F.aggStart;
+        lv[k].aggRows = F.aggRows;
+        lv[k].agg = L.agg;
+    }
+    TailLevel* p = nullptr;
+    AMG_TRY(amg_upload(c, d, &p, lv));
+    AMG_CUDA(cudaStreamSynchronize(c->stream));   // (lv ends here)
+    d->tailLevels = p;
+    return CF_OK;
+}
 
 constexpr int MW = MAXW_UNROLL;
 
@@ -605,6 +1006,38 @@ int launch_lanes(cf_context* c, AmgData* d, const AmgLevel& L, bool resid, const
     return CF_OK;
 }
 
+// Levels tailFrom.. of the V-cycle as one cluster launch.
+int launch_tail(cf_context* c, AmgData* d, int degree, const float* rf, float** result)
+{
+    const int from = d->tailFrom;
+    TailArgs a = {};
+    a.lv = static_cast<const TailLevel*>(d->tailLevels);
+    a.count = (int)d->lv.size() - from;
+    a.degree = degree;
+    a.rf = rf;
+    a.out = d->lv[from].x0;
+    a.inv = d->coarseInv;
+    a.scale = d->scale;
+    a.cc = c->d_chebC;
+    a.st = c->d_st;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = AMG_TAIL_CTAS;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(AMG_TAIL_CTAS);
+    cfg.blockDim = dim3(AMG_TAIL_T);
+    cfg.dynamicSmemBytes = (size_t)d->tailSmem;
+    cfg.stream = c->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    AMG_CUDA(cudaLaunchKernelEx(&cfg, ka_tail, a));
+    AMG_LAUNCH();
+    *result = a.out;
+    return CF_OK;
+}
+
 // Level l >= 1 of the V-cycle on its own buffers, from the residual rf of
 // level l - 1 (restricted here); returns the buffer holding the level's
 // correction, still to be prolonged by the caller.
@@ -615,6 +1048,7 @@ int vcycle_coarse(cf_context* c, AmgData* d, int l, int degree, const float* rf,
     cudaStream_t s = c->stream;
     const InnerState* st = c->d_st;
     const int last = (int)d->lv.size() - 1;
+    if (l == d->tailFrom && !c->amgLaunches) return launch_tail(c, d, degree, rf, result);
     if (l == last)
     {
         ka_restrict_coarse_solve<<<1, AMG_INV_THREADS, 0, s>>>(L.n, F.aggStart, F.aggRows, rf,
@@ -857,6 +1291,35 @@ int amg_prepare(cf_context* c, int coarsestCap, bool profile)
         C.A.ellW = H.uniformW;
         AMG_TRY(amg_alloc(c, d, &C.diag32, nagg));
         AMG_TRY(amg_alloc(c, d, &C.rD32, nagg));
+        if (nagg <= AMG_TAIL_ROWS)
+        {
+            C.tailCtas = nagg <= AMG_TAIL_WHOLE ? 1 : AMG_TAIL_CTAS;
+            const int tailM = (nagg + C.tailCtas * SLICE - 1) / (C.tailCtas * SLICE) * SLICE;
+            // (8 lanes of 4 rows read 32 banks: the width an odd multiple of 8)
+            int w = 1;
+            for (int s = 0; s < H.nslices; ++s)
+                w = std::max(w, (H.sliceOff[s + 1] - H.sliceOff[s]) / SLICE);
+            C.tailM = tailM;
+            C.tailW = (w + 7) / 8 * 8;
+            if (C.tailW / 8 % 2 == 0) C.tailW += 8;
+            const size_t size = (size_t)C.tailCtas * tailM * C.tailW;
+            std::vector<unsigned short> idx(size, 0xffffu);
+            std::vector<int> map((size_t)H.nnzp);
+            for (int s = 0; s < H.nslices; ++s)
+                for (int e = H.sliceOff[s]; e < H.sliceOff[s + 1]; ++e)
+                {
+                    const int q = e - H.sliceOff[s];
+                    const size_t at = (size_t)(s * SLICE + q % SLICE) * C.tailW + q / SLICE;
+                    map[e] = (int)at;
+                    if (H.col[e] != -1) idx[at] = (unsigned short)(H.col[e] & 0x7fffffff);
+                }
+            for (int k = 0; k <= C.tailCtas; ++k)
+                C.tailFine.push_back(aggStart[std::min(nagg, k * tailM)]);
+            AMG_TRY(amg_upload(c, d, &C.tailIdx, idx));
+            AMG_TRY(amg_upload(c, d, &C.tailMap, map));
+            AMG_TRY(amg_alloc(c, d, &C.tailVal, size));
+            AMG_CUDA(cudaMemsetAsync(C.tailVal, 0, sizeof(float) * size, c->stream));
+        }
         AMG_TRY(amg_alloc(c, d, &C.diag64, nagg));
         AMG_TRY(amg_alloc(c, d, &C.upper64, nfc));
         AMG_TRY(amg_alloc(c, d, &C.b, nagg));
@@ -891,6 +1354,7 @@ int amg_prepare(cf_context* c, int coarsestCap, bool profile)
                     "GAMG: the mesh does not coarsen to at most 128 cells (disconnected or "
                     "too few faces)");
     }
+    AMG_TRY(choose_tail(c, d));
     AMG_TRY(amg_alloc(c, d, &d->scale, 1));
     AMG_TRY(amg_alloc(c, d, &d->coarseInv, (size_t)Z.n * Z.n));
     AMG_CUDA(cudaStreamSynchronize(c->stream));
@@ -930,7 +1394,7 @@ int amg_stage(cf_context* c, int deflate, float scaleCorrection)
             (l == 0 && deflate) ? 1 : 0, upper, C.diag64, C.diag32, C.rD32);
         AMG_LAUNCH();
         ka_stage_vals<<<grid_n(c, (const void*)ka_stage_vals, C.nnzp), NT, 0, s>>>(
-            C.nnzp, C.eface, C.upper64, const_cast<float*>(C.A.val));
+            C.nnzp, C.eface, C.upper64, const_cast<float*>(C.A.val), C.tailMap, C.tailVal);
         AMG_LAUNCH();
     }
     AmgLevel& Z = d->lv.back();

@@ -135,7 +135,8 @@ struct cf_context
     int solves = 0;                        // cudaPCG solves on this topology so far
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
-    bool amgActive = false;                // inner PCG iterations use the V-cycle
+    bool amgActive = false;                // inner PCG iterations use the V-cycle ...
+    bool amgLaunches = false;              // ... with launches for every level (no cluster)
     int clusterShift = 10;                 // log2(rows per CTA) of the cluster PCG for this mesh
     double clusterRemote = 1.0;            // fraction of entries whose column lies in another CTA
     unsigned int* d_bar = nullptr;         // grid barrier of persistent inner solves: count, generation, error

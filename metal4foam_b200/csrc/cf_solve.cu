@@ -144,8 +144,9 @@ int launch_bicg_body(cf_context* c, cudaGraphConditionalHandle h, int useCond, i
 // the body sets the condition from the device-side convergence state.
 int get_graph(cf_context* c, int kind, int order, cudaGraphExec_t* out, int* bodyKernels)
 {
-    // (kind 2: PCG whose preconditioner is the multigrid V-cycle)
-    const auto key = std::make_pair(kind == 0 && c->amgActive ? 2 : kind, kind == 0 ? order : 1);
+    // (kind 2, 3: PCG whose preconditioner is the multigrid V-cycle)
+    const auto key = std::make_pair(kind == 0 && c->amgActive ? (c->amgLaunches ? 3 : 2) : kind,
+                                    kind == 0 ? order : 1);
     auto it = c->graphs.find(key);
     if (it != c->graphs.end())
     {
@@ -456,6 +457,7 @@ int solve_device(cf_context* c, int solver, double* psi_dev, const double* src_d
             CF_TRY(amg_prepare(c, o->nCellsInCoarsestLevel, o->profile != 0));
             CF_TRY(amg_stage(c, deflate ? 1 : 0, (float)o->scaleCorrection));
             c->amgActive = true;
+            c->amgLaunches = o->clusterMaxCells < 0;
         }
 
         // Chebyshev setup (metalFoamSolver.C:224-249); with GAMG the

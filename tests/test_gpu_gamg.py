@@ -308,3 +308,50 @@ def test_gamg_identical_with_either_stream(require_gpu, make):
         out.append((x, p.nIterations, p.finalResidual))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
     ctx.close()
+
+
+def random_links(n, seed):
+    """Seven random neighbours per cell: coarse rows of several hundred entries."""
+    rng = np.random.default_rng(seed)
+    a, b = np.repeat(np.arange(n), 4), rng.integers(0, n, 4 * n)
+    key = np.unique(np.minimum(a, b)[a != b] * n + np.maximum(a, b)[a != b])
+    low, upp = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    addr = mesh.ldu_addressing(n, low, upp)
+    upper = -rng.uniform(0.5, 2.0, addr.nf)
+    diag = 0.05 - (np.bincount(low, upper, n) + np.bincount(upp, upper, n))
+    return mesh.LduSystem("links", addr, diag, upper, None, rng.standard_normal(n), np.zeros(n))
+
+
+# the small levels as one cluster or with launches of their own: no level
+# below the coarsest, levels of a few rows per CTA, wide rows that leave
+# levels out, level sizes around the limit of 4,096 cells, a coarsest level of
+# 100 to 128 cells, another smoother degree
+@pytest.mark.parametrize("make,kw", [
+    (lambda: mesh.varcoeff3d((9, 8, 7), seed=51), {}),
+    (lambda: mesh.poisson2d(60, 50, seed=52), dict(nCellsInCoarsestLevel=4)),
+    (lambda: mesh.varcoeff3d((20, 19, 18), seed=53, permute=True), dict(nCellsInCoarsestLevel=12)),
+    (lambda: mesh.varcoeff3d((29, 28, 27), seed=54), dict(nSweeps=2)),
+    (lambda: mesh.varcoeff3d((31, 28, 27), seed=55, permute=True), dict(nSweeps=4)),
+    (lambda: mesh.prism3d((33, 31, 40), seed=56), dict(deflate="off")),
+    (lambda: mesh.poisson2d(300, 260, seed=57), dict(nCellsInCoarsestLevel=128)),
+    (lambda: random_links(9000, 58), {}),
+], ids=["one", "tiny", "cap12", "below", "above", "prism", "cap128", "wide"])
+def test_gamg_small_levels_in_a_cluster(require_gpu, make, kw):
+    """Every row is formed in the launches' order: the same solve bit for bit,
+    with fewer launches wherever there is a level to take in."""
+    s = make()
+    ctx = make_ctx(s)
+    out, launches = [], []
+    for cluster in (-1, 0, 0):
+        x = np.zeros(s.n)
+        l0 = ctx.kernel_launches()
+        p = ctx.solve(PCG, x, s.source, _lib.default_options(
+            preconditioner="GAMG", tolerance=1e-8, maxIter=300, clusterMaxCells=cluster, **kw))
+        launches.append(ctx.kernel_launches() - l0)
+        out.append((x, p.nIterations, p.finalResidual, p.finalResSum32))
+    taken = sum(n <= 2000 for n in ctx.gamg_levels()[1:-1])
+    ctx.close()
+    for x, *rest in out[1:]:
+        assert np.array_equal(x, out[0][0]) and tuple(rest) == out[0][1:]
+    if taken and s.addr.nf < 3 * s.n + 1:       # (not where the rows may be too wide)
+        assert launches[2] < launches[0]
