@@ -95,7 +95,11 @@ namespace {
 constexpr int RES_MAX_PARTS = 256;   // CTAs of one system at most
 constexpr int RES_MAX_ROWS = 6144;   // rows of a part at most (the last entry of CHIP)
 constexpr int RES_COPIES = 8;        // copies of every reduction word
-constexpr size_t RES_RED_WORDS = (size_t)RES_COPIES * RES_MAX_PARTS * 4;
+// A part's words have a 128-byte line of their own (with four parts to a line,
+// whose writers and pollers meet in L2: 64^3 Jacobi 8.66 us per iteration, 8.29
+// so; prism 200K order 8 18.1 and 17.6).
+constexpr int RES_STRIDE = 16;       // 8-byte words
+constexpr size_t RES_RED_WORDS = (size_t)RES_COPIES * RES_MAX_PARTS * RES_STRIDE;
 constexpr int RES_HQ = 4;            // halo slots a thread keeps in registers
 
 struct ResArgs
@@ -252,7 +256,7 @@ __device__ __forceinline__ void red_send(double (&v)[NR], u64* red, int rank, un
         for (int r = 0; r < NR; ++r) t[r] = warp_sum(lane < (T >> 5) ? sh.red[r][lane] : 0.0);
         if (lane < RES_COPIES)
         {
-            u64* w = red + ((size_t)lane * RES_MAX_PARTS + rank) * 4;
+            u64* w = red + ((size_t)lane * RES_MAX_PARTS + rank) * RES_STRIDE;
 #pragma unroll
             for (int r = 0; r < NR; ++r) st_double(w + 2 * r, t[r], epoch);
         }
@@ -273,7 +277,7 @@ __device__ __forceinline__ void red_recv(const ResArgs& a, const u64* red, int r
     for (int r = 0; r < NR; ++r) acc[r] = 0.0;
     for (int p = tid; p < a.nparts; p += T)
     {
-        const u64* w = red + ((size_t)(rank % RES_COPIES) * RES_MAX_PARTS + p) * 4;
+        const u64* w = red + ((size_t)(rank % RES_COPIES) * RES_MAX_PARTS + p) * RES_STRIDE;
         u64 f[NR][2];
 #pragma unroll
         for (int r = 0; r < NR; ++r) ld_words(w + 2 * r, f[r][0], f[r][1]);
