@@ -7,6 +7,8 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -38,16 +40,26 @@ def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every .cu of csrc/ into libcudafoam.so for sm_100a."""
     if not force and not _stale():
         return LIB
-    cmd = [NVCC, "-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC", "-shared",
-           "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-o", LIB + ".tmp", *sources()]
+    flags = ["-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC",
+             "-I", os.path.join(ROOT, "include"), "-I", CSRC]
     if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("nvcc failed building libcudafoam.so")
-    if verbose:
-        sys.stderr.write(res.stderr)
+        flags.insert(0, "-Xptxas=-v")
+
+    def run(cmd):
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            sys.stderr.write(res.stdout + res.stderr)
+            raise RuntimeError("nvcc failed building libcudafoam.so")
+        if verbose:
+            sys.stderr.write(res.stderr)
+
+    # one compiler per file at a time on every core, then the link
+    with tempfile.TemporaryDirectory() as tmp:
+        objs = [os.path.join(tmp, os.path.basename(s) + ".o") for s in sources()]
+        with ThreadPoolExecutor(max(1, min(16, os.cpu_count() or 1))) as pool:
+            list(pool.map(run, [[NVCC, *flags, "-c", "-o", o, s]
+                                for o, s in zip(objs, sources())]))
+        run([NVCC, *ARCH, "-Xcompiler", "-fPIC", "-shared", "-o", LIB + ".tmp", *objs])
     os.replace(LIB + ".tmp", LIB)
     return LIB
 
