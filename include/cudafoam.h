@@ -207,9 +207,10 @@ int cf_context_set_stream(cf_context* ctx, void* stream);
  * for meshes above 65536 cells).  Results are returned in the caller's
  * ordering either way. */
 int cf_context_set_reorder(cf_context* ctx, int32_t mode);
-/* Polls a bounded device-side wait of this context (the grid barriers of
- * persistent inner solves, persistentMaxCells) makes before it gives up;
- * a wait that gives up ends the kernel and the solve returns
+/* Polls a bounded device-side wait of this context makes before it gives
+ * up, which ends the kernel.  A resident inner solve (clusterMaxCells) then
+ * runs through the graph loop instead; with the grid barriers of persistent
+ * inner solves (persistentMaxCells) the solve returns
  * CF_ERR_DEVICE_TIMEOUT, leaving the context usable.  0 restores the
  * default, 2^24 polls of about 64 ns each.  No reference counterpart. */
 int cf_context_set_wait_limit(cf_context* ctx, int64_t polls);

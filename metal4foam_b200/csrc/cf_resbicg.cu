@@ -54,7 +54,7 @@ typedef unsigned long long u64;
 
 constexpr int RSB_MAX_R = 24;        // 256-row groups per CTA at most
 constexpr int RSB_MAX_CTAS = 256;
-constexpr int RSB_ABOVE = NT * 160;  // rows up to which cf_clubicg.cu takes the mesh
+constexpr int RSB_ABOVE = NT * 160;  // rows that fit one cluster (cf_clubicg.cu)
 constexpr int RSB_COPIES = 8;        // copies of words every CTA polls
 // A flag has a 128-byte line of its own (in lines of 8 or 32 flags, whose
 // writers and pollers meet in L2, a barrier takes 3 to 7 us instead of about
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_bicg(const __grid_constant__ ResB
 
 // groups per CTA the kernels are compiled for
 const int RSB_ROWS[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 18, 20, 22, 24};
-constexpr int RSB_TEAM_R = 10;        // for several systems
+constexpr int RSB_TEAM_R = 10;        // for several systems (15 registers per group of rows)
 
 template <int W>
 const void* kernel_r(int R)
