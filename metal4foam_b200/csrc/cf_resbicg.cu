@@ -878,7 +878,8 @@ int res_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagL
 {
     *ran = false;
     res_bicg_prepare(c);
-    if (maxIter <= 0 || !c->resBicg) return CF_OK;
+    // (the plan may be older than a switch to the 32-bit column stream)
+    if (maxIter <= 0 || !c->resBicg || !sell_of(c).pval) return CF_OK;
     const InnerRun run = inner_run(c, nullptr, target, maxIter, ips, 1, stagLimit);
     if (c->resBicgTeam) return c->resBicgTeam->solve(c, run, ran);
     // one resident launch at a time on the device: other solves go through

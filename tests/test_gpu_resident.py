@@ -339,3 +339,31 @@ def test_resident_from_two_threads(require_gpu):
         for x, p, _ in out[k]:
             assert np.array_equal(x, ref[k][0]) and p.nIterations == ref[k][1].nIterations
         ctxs[k].close()
+
+
+def test_bicgstab_with_the_other_column_stream(require_gpu):
+    """A switch to 32-bit columns (and back) after a resident solve: the
+    graph loop on that stream, alone and for several components."""
+    s = mesh.upwind3d((40, 36, 31), seed=30)
+    ctx = _lib.Context(0)
+    ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
+    ctx.set_coeffs(s.diag, s.upper, s.lower)
+    b = np.random.default_rng(31).standard_normal((2, s.n))
+    launches = {}
+    for bits in (16, 32, 16):
+        ctx.set_spmv_config(indexBits=bits)
+        out = []
+        for cluster in (-1, 0):
+            x = np.zeros(s.n)
+            l0 = ctx.kernel_launches()
+            opts = _lib.default_options(tolerance=1e-8, maxIter=2000, clusterMaxCells=cluster)
+            p = ctx.solve(_lib.CF_SOLVER_PBICGSTAB, x, s.source, opts)
+            launches[bits, cluster] = ctx.kernel_launches() - l0
+            psi = np.zeros((2, s.n))
+            q = ctx.solve_multi(_lib.CF_SOLVER_PBICGSTAB, psi, b, opts)
+            assert p.converged and all(r.converged for r in q)
+            out.append((x, psi, p.nIterations, [r.nIterations for r in q]))
+        assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+        assert out[0][2:] == out[1][2:]
+    assert launches[16, 0] < launches[16, -1] and launches[32, 0] == launches[32, -1]
+    ctx.close()
