@@ -367,3 +367,46 @@ def test_bicgstab_with_the_other_column_stream(require_gpu):
         assert out[0][2:] == out[1][2:]
     assert launches[16, 0] < launches[16, -1] and launches[32, 0] == launches[32, -1]
     ctx.close()
+
+
+def test_bicgstab_components_on_several_threads(require_gpu):
+    """Two multi-RHS solves and a cudaPCG solve at once: their launches take
+    turns on the SMs, every result is the one of the graph loop."""
+    ms = [mesh.upwind3d((40, 36, 31), seed=32), mesh.upwind3d((48, 45, 40), seed=33)]
+    sp = mesh.varcoeff3d((40, 40, 22), seed=34, permute=True)
+    ctxs = []
+    for s in ms:
+        ctx = _lib.Context(0)
+        ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
+        ctx.set_coeffs(s.diag, s.upper, s.lower)
+        ctxs.append(ctx)
+    cp = context(sp)
+    b = [np.random.default_rng(35 + k).standard_normal((3, s.n)) for k, s in enumerate(ms)]
+
+    def multi(k, cluster):
+        psi = np.zeros((3, ms[k].n))
+        p = ctxs[k].solve_multi(_lib.CF_SOLVER_PBICGSTAB, psi, b[k], _lib.default_options(
+            tolerance=1e-8, maxIter=2000, clusterMaxCells=cluster))
+        return psi, [q.nIterations for q in p]
+
+    ref = [multi(k, -1) for k in range(2)]
+    for _ in range(2):
+        refp = solve(cp, sp, -1)
+    out = [[], [], []]
+
+    def work(k):
+        for _ in range(4):
+            out[k].append(multi(k, 0) if k < 2 else solve(cp, sp))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(2):
+        assert len(out[k]) == 4
+        for psi, its in out[k]:
+            assert np.array_equal(psi, ref[k][0]) and its == ref[k][1]
+        ctxs[k].close()
+    assert len(out[2]) == 4 and all(np.array_equal(x, refp[0]) for x, _, _ in out[2])
+    cp.close()
