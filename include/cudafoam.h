@@ -123,7 +123,13 @@ typedef struct
                                   to what the SMs hold (about 900,000 cells)
                                   as one cooperative launch with the mesh
                                   split over the SMs; the split is made by
-                                  the third solve on a topology.
+                                  the third solve on a topology.  The forms
+                                  of cudaPCG add their FP64 sums in orders of
+                                  their own: results agree up to FP32
+                                  roundings of alpha and beta, and nearly
+                                  always to the bit; which form runs depends
+                                  on the context, its solves so far and
+                                  these options, not on other threads.
                                   cudaPBiCGStab: meshes of up to 40960 cells
                                   with at most 6 neighbours per cell in one
                                   cluster, larger ones up to 6144 cells per
@@ -569,8 +575,11 @@ int cf_autotune(cf_context* ctx, int32_t reps, int32_t apply, cf_spmv_config* be
  * otherwise); all pointers are device pointers on it; work queued earlier on
  * any stream of that device completes first, and everything is complete on
  * return.  Every
- * system gets exactly what cf_solve_device on it alone returns.  A context
- * may appear once.  No counterpart in the reference. */
+ * system gets exactly what cf_solve_device on it alone returns; with
+ * streams >= 4 and at least 4 systems, cudaPCG systems of more than 384 and at
+ * most 1216 cells per SM (57K to 180K on B200) get what it returns with
+ * clusterMaxCells < 0.  A context may appear once.  No counterpart in the
+ * reference. */
 int cf_solve_many_device(cf_context* const* ctx, int32_t count, int32_t solver,
                          double* const* psi, const double* const* source,
                          const double* const* diag, const double* const* upper,

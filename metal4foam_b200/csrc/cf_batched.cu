@@ -1517,15 +1517,16 @@ int whole_build(cf_batch* bt, int reorder)
     return CF_OK;
 }
 
-// The inner solves of all active systems, each run whole.  *ran stays false
-// when another resident launch has the device or a wait gave up (the states
-// are then as kb_outer_begin left them): the batched loop runs instead.
+// The inner solves of all active systems, each run whole, after the resident
+// launches of other threads on the device.  *ran stays false when a wait gave
+// up (the states are then as kb_outer_begin left them): the batched loop runs
+// instead.
 int whole_loop(cf_batch* bt, const cf_options* o, bool* ran)
 {
     *ran = false;
     cudaStream_t s = bt->stream;
     std::unique_lock<std::mutex> turn(res_device_lock(bt->device), std::defer_lock);
-    if (!bt->slots.empty() && !turn.try_lock()) return CF_OK;
+    if (!bt->slots.empty()) turn.lock();
     const int order = o->chebyshevOrder;
     if (bt->wholeOrder != order)
     {

@@ -133,6 +133,7 @@ struct cf_context
     bool resBicgShared = false;            // (a clone's: its source's)
     cf::ResBicgTeam* resBicgTeam = nullptr; // clones that run their inner solves together
     int solves = 0;                        // cudaPCG solves on this topology so far
+    int concurrent = 1;                    // solves that cf_solve_many_device runs side by side
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
     bool amgActive = false;                // inner PCG iterations use the V-cycle ...
@@ -299,10 +300,25 @@ int persistent_status(cf_context* c);
 // it takes the host as long as 5 to 10 solves save (25 ms at 300K cells), so a
 // mesh that is solved on once or twice does without.  resident_inner runs and
 // completes one inner solve (state in h_st and d_st, the returned correction
-// in d_D) when there is a split and no other resident launch of the process
-// runs on the device; *ran tells whether it did.
+// in d_D) when there is a split, after the resident launches of other threads
+// on the device; *ran tells whether it did.
+//
+// It waits for its turn because its FP64 sums fold in another order than the
+// graph loop's: whether it runs must not depend on what other threads do.
+// Solves that take turns are also faster than graph loops side by side, but
+// for many systems of one medium size: 2, 3, 4, 8 at once, ms, turns / graph
+// loops: 50K cells 2.6 / 3.9, 3.7 / 4.5, 4.9 / 5.1, 9.7 / 9.9; 74K -, 4.0 / 3.7,
+// 5.2 / 4.0, 10.1 / 7.5; 110K 3.0 / 3.9, 4.3 / 4.2, 5.7 / 4.7, 11.2 / 9.1; 149K -,
+// 4.9 / 5.3, 6.4 / 5.8, 12.5 / 11.2; 195K -, 5.1 / 5.9, 6.7 / 6.8, 13.4 / 13.6;
+// 262K 3.8 / 5.9, 5.7 / 7.4, 7.6 / 8.9, 15.1 / 18.0; 885K 15 / 18, 23 / 28,
+// 32 / 41, 64 / 84.  So cf_solve_many_device with at least
+// RESIDENT_BESIDE systems side by side gives those of more than
+// RESIDENT_BESIDE_MIN and at most RESIDENT_BESIDE_MAX rows per SM to graph loops.
 constexpr int RESIDENT_MIN_ROWS_PER_SM = 128;
 constexpr int RESIDENT_AFTER_SOLVES = 2;
+constexpr int RESIDENT_BESIDE = 4;
+constexpr int RESIDENT_BESIDE_MIN = 384;
+constexpr int RESIDENT_BESIDE_MAX = 1216;
 constexpr int RESIDENT_MAX_ROWS = 1 << 20;   // no device holds more on its SMs
 struct InnerRun;
 InnerRun inner_run(const cf_context* c, const double* mean, double target, int maxIter, int ips,

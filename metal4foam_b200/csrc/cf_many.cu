@@ -4,7 +4,8 @@
 // + cf_solve_device, unchanged).  Small systems fill few SMs and their
 // kernels are short; on separate streams their launches and host
 // synchronisations overlap.  Every system gets exactly what cf_solve_device
-// on it alone returns (same kernels, same grids, same order of reductions).
+// on it alone returns: same kernels, same grids, same order of reductions (the
+// graph loop's where cf_host.hpp, RESIDENT_BESIDE, chooses it).
 #include "cudafoam.h"
 #include "cf_host.hpp"
 
@@ -81,11 +82,13 @@ extern "C" int cf_solve_many_device(cf_context* const* ctx, int32_t count, int32
             cf_context* c = ctx[i];
             cudaStream_t saved = c->stream;
             c->stream = st[w];
+            c->concurrent = W;
             int r = CF_OK;
             if (diag) r = cf_set_coeffs_device(c, diag[i], upper[i], lower ? lower[i] : nullptr);
             if (r == CF_OK) r = cf_solve_device(c, solver, psi[i], source[i], opts, &perf[i]);
             if (r != CF_OK) msg[i] = cf_last_error();
             c->stream = saved;
+            c->concurrent = 1;
             rc[i] = r;
         }
     };

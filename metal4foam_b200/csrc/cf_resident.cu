@@ -869,6 +869,9 @@ int resident_inner(cf_context* c, const double* mean, double target, int maxIter
     if (maxIter <= 0 || c->solves < RESIDENT_AFTER_SOLVES ||
         c->n < RESIDENT_MIN_ROWS_PER_SM * c->numSMs || c->maxRowLen < 4)
         return CF_OK;
+    if (c->concurrent >= RESIDENT_BESIDE && c->n > RESIDENT_BESIDE_MIN * c->numSMs &&
+        c->n <= RESIDENT_BESIDE_MAX * c->numSMs)
+        return CF_OK;
     if (!c->residentTried)
     {
         c->residentTried = true;
@@ -876,9 +879,7 @@ int resident_inner(cf_context* c, const double* mean, double target, int maxIter
     }
     const ResPlan* p = static_cast<const ResPlan*>(c->resident);
     if (!p) return CF_OK;
-    // (another resident launch on the device: the graph path)
-    std::unique_lock<std::mutex> turn(res_device_lock(c->device), std::try_to_lock);
-    if (!turn.owns_lock()) return CF_OK;
+    std::lock_guard<std::mutex> turn(res_device_lock(c->device));
     cudaStream_t s = c->stream;
     const int rc = res_launch(p, inner_run(c, mean, target, maxIter, ips, order, stagLimit), s);
     if (rc != CF_OK) return rc;

@@ -72,7 +72,8 @@ int res_plan_build(int device, int n, const HostLayout& L, bool ordered, int npa
                    long long entOff, int rowOff, cudaStream_t s, ResPlan** plan);
 void res_plan_free(ResPlan* plan);
 // The waits of a resident launch need all its CTAs on the device: launches
-// run under this lock, with at most one CTA per SM in all.
+// run under this lock until they have ended, with at most one CTA per SM in
+// all.
 std::mutex& res_device_lock(int device);
 int res_launch(const ResPlan* plan, const InnerRun& run, cudaStream_t s);
 // fresh exchange words after a wait has given up
