@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <map>
 #include <string>
 #include <thread>
@@ -323,6 +324,8 @@ constexpr int RESIDENT_MAX_ROWS = 1 << 20;   // no device holds more on its SMs
 struct InnerRun;
 InnerRun inner_run(const cf_context* c, const double* mean, double target, int maxIter, int ips,
                    int order, int stagLimit);
+// solves under way on a device of this process
+std::atomic<int>& res_in_flight(int device);
 void resident_release(cf_context* c);
 int resident_inner(cf_context* c, const double* mean, double target, int maxIter, int ips,
                    int order, int stagLimit, bool* ran);

@@ -610,6 +610,7 @@ __global__ void __launch_bounds__(NT, 1) k_res_bicg(const __grid_constant__ ResB
 
 // groups per CTA the kernels are compiled for
 const int RSB_ROWS[] = {2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 18, 20, 22, 24};
+constexpr int RSB_TURNS_ABOVE = 2560; // rows per SM from which solves side by side take turns
 constexpr int RSB_TEAM_R = 10;        // for several systems (15 registers per group of rows)
 
 template <int W>
@@ -882,10 +883,23 @@ int res_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagL
     if (maxIter <= 0 || !c->resBicg || !sell_of(c).pval) return CF_OK;
     const InnerRun run = inner_run(c, nullptr, target, maxIter, ips, 1, stagLimit);
     if (c->resBicgTeam) return c->resBicgTeam->solve(c, run, ran);
-    // one resident launch at a time on the device: other solves go through
-    // the graph loop meanwhile
-    std::unique_lock<std::mutex> turn(res_device_lock(c->device), std::try_to_lock);
-    if (!turn.owns_lock()) return CF_OK;
+    // One resident launch at a time on the device; the others wait or go
+    // through the graph loop, which gives the same bits.  A launch of two
+    // groups of rows per SM leaves room for graph loops beside it; of the
+    // larger meshes, which do not, two take turns and more keep the graph loop
+    // each, until it needs HBM.  ms, in turns / a launch beside graph loops /
+    // graph loops only: 50K cells 3 at once 10.3 / 6.9 / 8.8, 8 at once 31 / 19 /
+    // 24; 110K 2: 7.1 / 9.6 / 8.2, 3: 11.8 / 13.6 / 10.9, 8: 36 / 30 / 24; 262K 2:
+    // 12.1 / 13.0 / 15.1, 3: 18.1 / 18.9 / 17.0, 8: 55 / 56 / 53; 405K 3: 22 / 26 /
+    // 22, 8: 69 / 70 / 66; 593K 3: 26 / 33 / 31, 8: 76 / 83 / 85; 885K 2: 23 / 31 / 33,
+    // 8: 105 / 115 / 135.
+    const int rows = c->n / c->numSMs;
+    const int beside = std::max(c->concurrent, res_in_flight(c->device).load());
+    std::unique_lock<std::mutex> turn(res_device_lock(c->device), std::defer_lock);
+    if (beside <= 2 || rows > RSB_TURNS_ABOVE)
+        turn.lock();
+    else if (rows > 2 * NT || !turn.try_lock())
+        return CF_OK;
     return launch(&c, &run, 1, ran);
 }
 

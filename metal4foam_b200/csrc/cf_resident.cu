@@ -53,6 +53,7 @@
 #include "cf_cluster_ll.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -650,6 +651,7 @@ __global__ void __launch_bounds__(TB, 1) k_res_chip(const __grid_constant__ ResA
 // ------------------------------------------------------------------- host
 
 std::mutex g_resident[64];
+std::atomic<int> g_inFlight[64];
 
 // The kernels: R rows per thread, RM of them with their matrix entries in
 // registers, at most TB threads.  In order of preference; the first whose
@@ -686,6 +688,7 @@ int up(ResPlan* p, T** d, const T* h, size_t count, cudaStream_t s)
 }  // namespace
 
 std::mutex& res_device_lock(int device) { return g_resident[device & 63]; }
+std::atomic<int>& res_in_flight(int device) { return g_inFlight[device & 63]; }
 
 void res_plan_free(ResPlan* p)
 {

@@ -391,6 +391,12 @@ int solve_device(cf_context* c, int solver, double* psi_dev, const double* src_d
 {
     const bool bicg = solver == CF_SOLVER_PBICGSTAB;
     const char* name = bicg ? "cudaPBiCGStab" : "cudaPCG";
+    struct InFlight
+    {
+        std::atomic<int>& count;
+        explicit InFlight(std::atomic<int>& n) : count(n) { ++count; }
+        ~InFlight() { --count; }
+    } inFlight(res_in_flight(c->device));
     cudaStream_t s = c->stream;
     const int n = c->n;
     const DevSell A = sell_of(c);

@@ -148,3 +148,23 @@ def test_many_pcg_takes_one_form(require_gpu, rows, count, split):
             assert np.array_equal(x, a if split else g, equal_nan=True)
     for c in ctxs:
         c.close()
+
+
+# momentum systems of two and three 256-row groups per SM and of more than
+# 2,560 rows per SM; the same bits in every form, told apart by their launches
+@pytest.mark.parametrize("rows,count,form", [(520, 2, "whole"), (520, 3, "loop"),
+                                             (2561, 3, "whole")])
+def test_many_bicgstab_forms(require_gpu, rows, count, form):
+    import torch
+    m = torch.cuda.get_device_properties(0).multi_processor_count
+    ss = [mesh.upwind3d((m, rows), seed=40 + k) for k in range(count)]
+    ctxs = [context(s) for s in ss]
+    kw = dict(tolerance=1e-6, maxIter=40, maxRestarts=1)
+    ref, loop, _ = many(ctxs, ss, _lib.CF_SOLVER_PBICGSTAB,
+                        _lib.default_options(clusterMaxCells=-1, **kw))
+    xs, launches, _ = many(ctxs, ss, _lib.CF_SOLVER_PBICGSTAB, _lib.default_options(**kw))
+    for x, r, a, b in zip(xs, ref, launches, loop):
+        assert np.array_equal(x, r)
+        assert (a < b) if form == "whole" else (a == b), (a, b)
+    for c in ctxs:
+        c.close()
