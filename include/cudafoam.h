@@ -123,7 +123,9 @@ typedef struct
                                   to what the SMs hold (about 900,000 cells)
                                   as one cooperative launch with the mesh
                                   split over the SMs; the split is made by
-                                  the third solve on a topology.  The forms
+                                  the third solve on a topology (by the first
+                                  for one cluster, up to 8192 cells or four
+                                  neighbours per cell).  The forms
                                   of cudaPCG add their FP64 sums in orders of
                                   their own: results agree up to FP32
                                   roundings of alpha and beta, and nearly

@@ -47,6 +47,8 @@ namespace {
 
 constexpr int CLB_MAX_R = 10;                              // 256-row blocks of a CTA at most
 constexpr int CLB_BLOCKS = CLU_MAX_CTAS * CLB_MAX_R;       // of the mesh
+constexpr int CLB_FIRST_ROWS = 32768;                      // for a first solve
+constexpr int CLB_FIRST_HALO = 2560;
 // reduction values: rA0.AyA | sum|s|, s.t, t.t | sum|r|, rA0.r
 constexpr int CLB_VALUES = 6;
 
@@ -405,9 +407,15 @@ void clu_bicg_release(cf_context* c)
     c->cluBicgTried = c->cluBicgShared = false;
 }
 
-void clu_bicg_prepare(cf_context* c)
+void clu_bicg_prepare(cf_context* c, bool first)
 {
     if (c->cluBicgTried) return;
+    // A mesh of more than 32,768 cells, or one numbered so that the blocks read
+    // most of the others, gains little next to the 2 to 3 ms that its split takes
+    // the host (39K cells in natural order, first solve: 5.1 ms without, 6.8
+    // with; 22K scattered 4.9 and 7, 12K 4.4 and 4.4).  Others gain more at once
+    // than it takes (12K in natural order 4.0 and 2.2, 22K 5.0 and 3.3).
+    if (first && c->n > CLB_FIRST_ROWS) return;
     c->cluBicgTried = true;
     if (c->hostSliceOff.empty() || c->maxRowLen > 6 || c->n > NT * CLB_BLOCKS) return;
     // the graph loop's kernels run one row per thread on these blocks
@@ -428,7 +436,12 @@ void clu_bicg_prepare(cf_context* c)
     ResHost H;
     try
     {
-        if (!res_blocks(c->n, host_layout(c), per * NT, H, 4)) return;
+        if (!res_blocks(c->n, host_layout(c), per * NT, H, 4,
+                        first ? CLB_FIRST_HALO : CLU_MAX_HALO))
+        {
+            c->cluBicgTried = !first;
+            return;
+        }
     }
     catch (...)
     {
@@ -444,7 +457,7 @@ int clu_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagL
 {
     *ran = false;
     if (maxIter <= 0) return CF_OK;
-    clu_bicg_prepare(c);
+    clu_bicg_prepare(c, c->bicgSolves == 0);
     const CluPlan* p = static_cast<const CluPlan*>(c->cluBicg);
     if (!p) return CF_OK;
     cudaStream_t s = c->stream;

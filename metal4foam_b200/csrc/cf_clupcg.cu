@@ -474,7 +474,7 @@ int clu_plan_upload(ResHost& H, int ctas, int buffers, int nd, long long entOff,
             }
         // columns in the common layout
         const int zero = H.maxLocP + 2 * halo;
-        if (zero > 65535 || halo > 8191) return CF_OK;
+        if (zero > 65535 || halo > CLU_MAX_HALO) return CF_OK;
         for (const ResPart& q : H.parts)
             for (long long e = (long long)q.rowBase * W; e < ((long long)q.rowBase + q.nlocP) * W; ++e)
             {

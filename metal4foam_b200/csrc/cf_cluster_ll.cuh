@@ -19,6 +19,7 @@ namespace cf {
 typedef unsigned long long u64;
 
 constexpr int CLU_MAX_CTAS = 16;
+constexpr int CLU_MAX_HALO = 8191;   // halo values of a part at most
 constexpr unsigned int CLU_NONE = 0xffffffffu;
 
 // Every part has the same shared-memory layout of a gathered vector, in

@@ -92,7 +92,7 @@ void free_topology(cf_context* c)
     clu_release(c);
     clu_bicg_release(c);
     res_bicg_release(c);
-    c->solves = 0;
+    c->solves = c->bicgSolves = 0;
     c->hostCol.clear();
     c->hostSliceOff.clear();
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);

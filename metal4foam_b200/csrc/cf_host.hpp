@@ -134,6 +134,7 @@ struct cf_context
     bool resBicgShared = false;            // (a clone's: its source's)
     cf::ResBicgTeam* resBicgTeam = nullptr; // clones that run their inner solves together
     int solves = 0;                        // cudaPCG solves on this topology so far
+    int bicgSolves = 0;                    // cudaPBiCGStab solves on it
     int concurrent = 1;                    // solves that cf_solve_many_device runs side by side
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;
@@ -271,12 +272,15 @@ int cluster_inner(cf_context* c, int order, int maxCells, bool* ran);
 // CLU_MAX_ROWS cells, matrix and vectors in registers (cf_clupcg.cu); runs
 // and completes the inner solve as resident_inner does.
 constexpr int CLU_MAX_ROWS = 40960;
+constexpr int CLU_FIRST_ROWS = 8192;
 int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int ips, int order,
               int stagLimit, bool* ran);
 void clu_release(cf_context* c);
 // The inner BiCGStab of a small mesh in one cluster (cf_clubicg.cu), the graph
-// loop's result bit for bit; _prepare makes the split (once per topology).
-void clu_bicg_prepare(cf_context* c);
+// loop's result bit for bit; _prepare makes the split (once per topology;
+// `first`: by its first solve, which does without where it costs more than it
+// gives).
+void clu_bicg_prepare(cf_context* c, bool first);
 int clu_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagLimit, bool* ran);
 void clu_bicg_release(cf_context* c);
 // The same for larger meshes as one cooperative launch (cf_resbicg.cu).

@@ -1011,7 +1011,7 @@ int solve_multi_streams(cf_context* c, int32_t solver, int32_t nrhs, double* psi
     // the FP32 operator in BiCGStab's form, staged once on the shared arrays
     const int wantSym32 = c->hasLower ? 0 : 1;
     if (wantSym32 != c->val32Sym) CF_TRY(stage_vals(c, wantSym32));
-    clu_bicg_prepare(c);   // (the clones share the split)
+    clu_bicg_prepare(c, false);   // (the clones share the split)
     res_bicg_prepare(c);
     for (int w = 0; w < W; ++w) CF_TRY(context_clone_sync(c, c->clones[w]));
     // the clones' streams start after the work queued so far on this one

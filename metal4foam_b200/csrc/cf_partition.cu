@@ -286,24 +286,42 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
         try
         {
             std::vector<int32_t> h;
+            std::vector<int32_t> pos((size_t)R.slots, -1);   // halo value of a slot
             for (;;)
             {
                 const int p = nextPart.fetch_add(1);
                 if (p >= nparts) return;
                 ResPart& P = R.parts[p];
                 h.clear();
+                int lo = R.slots, hi = -1;
                 for (int l = 0; l < P.nb; ++l)
                 {
                     const int r = R.rowMap[(size_t)P.rowBase + l];
                     for (int q = g.start[r]; q < g.start[r + 1]; ++q)
                     {
                         const int c = g.adj[q];
-                        if (part[c] != p) h.push_back(R.parts[part[c]].llBase + loc[c]);
+                        if (part[c] == p) continue;
+                        const int s = R.parts[part[c]].llBase + loc[c];
+                        if (pos[s] >= 0) continue;
+                        pos[s] = 0;
+                        h.push_back(s);
+                        lo = std::min(lo, s);
+                        hi = std::max(hi, s);
                     }
                 }
-                std::sort(h.begin(), h.end());
-                h.erase(std::unique(h.begin(), h.end()), h.end());
                 P.nh = (int)h.size();
+                // in ascending order: sorted, or (many of few) picked up in it
+                if (P.nh > (hi - lo) / 16)
+                {
+                    int k = 0;
+                    for (int s = lo; s <= hi; ++s)
+                        if (pos[s] >= 0) h[k++] = s;
+                }
+                else
+                {
+                    std::sort(h.begin(), h.end());
+                }
+                for (int k = 0; k < P.nh; ++k) pos[h[k]] = k;
                 if (P.nlocP + P.nh + 1 > 65535)
                 {
                     fits = false;
@@ -332,16 +350,14 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
                                 R.idx[at] = (uint16_t)loc[c];
                             else
                                 R.idx[at] = (uint16_t)(P.nlocP +
-                                                       (std::lower_bound(h.begin(), h.end(),
-                                                                         R.parts[part[c]].llBase +
-                                                                             loc[c]) -
-                                                        h.begin()));
+                                                       pos[R.parts[part[c]].llBase + loc[c]]);
                             R.emap[at] = e;
                             ++k;
                         }
                     }
                     for (; k < W; ++k) R.idx[(size_t)pair_index(sb, W, k, lane)] = zero;
                 }
+                for (int s : h) pos[s] = -1;
                 halo[p] = h;
             }
         }
@@ -350,8 +366,10 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
             fits = false;   // out of memory: no split
         }
     };
+    // (the longest part: several threads also where the others take one)
+    const int workers = n < 4096 ? nt : std::max(nt, 4);
     std::vector<std::thread> pool;
-    for (int t = 1; t < nt; ++t)
+    for (int t = 1; t < workers; ++t)
     {
         try
         {
@@ -378,7 +396,7 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
 
 // Consecutive ranges of rowsPerPart rows (whole slices), rows in the internal
 // order; the exchange slot of a row is the row itself.
-bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int width)
+bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int width, int maxHalo)
 {
     const int W = std::max(width, (int)L.maxw);
     if (W < 1 || W > 8 || rowsPerPart < SLICE || rowsPerPart % SLICE || n < 1) return false;
@@ -392,7 +410,12 @@ bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int wid
     R.idx.resize((size_t)R.rowsP * W);
     R.emap.assign((size_t)R.rowsP * W, -1);
     R.haloSlot.clear();
-    std::vector<int32_t> h;
+    // local index of every column of the part at hand; the halo columns are
+    // marked and then numbered in ascending order, so cells numbered at
+    // random cost little more than others (12K cells: 1.2 ms, 8.9 with the halo
+    // sorted and searched; 0.4 and 1.2 in natural order)
+    constexpr int32_t NONE = -1, HALO = -2;
+    std::vector<int32_t> local((size_t)n, NONE);
     for (int p = 0; p < nparts; ++p)
     {
         ResPart& P = R.parts[p];
@@ -410,19 +433,25 @@ bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int wid
                 if (L.col[e] != -1) fn(e, L.col[e] & 0x7fffffff);
             }
         };
-        h.clear();
+        for (int l = 0; l < P.nloc; ++l) local[r0 + l] = l;
+        int lo = n, hi = -1;
         for (int r = r0; r < r0 + P.nloc; ++r)
             each(r, [&](int, int c) {
-                if (c < r0 || c >= r0 + P.nloc) h.push_back(c);
+                if (local[c] != NONE) return;
+                local[c] = HALO;
+                lo = std::min(lo, c);
+                hi = std::max(hi, c);
             });
-        std::sort(h.begin(), h.end());
-        h.erase(std::unique(h.begin(), h.end()), h.end());
-        P.nh = (int)h.size();
         P.haloBase = (int)R.haloSlot.size();
-        R.haloSlot.insert(R.haloSlot.end(), h.begin(), h.end());
+        for (int c = lo; c <= hi; ++c)
+            if (local[c] == HALO)
+            {
+                local[c] = P.nlocP + P.nh++;
+                R.haloSlot.push_back(c);
+            }
         R.maxLocP = std::max(R.maxLocP, P.nlocP);
         R.maxHalo = std::max(R.maxHalo, P.nh);
-        if (P.nlocP + P.nh + 1 > 65535) return false;
+        if (P.nh > maxHalo || P.nlocP + P.nh + 1 > 65535) return false;
         for (int l = 0; l < P.nlocP; ++l)
         {
             const long long sb = ((long long)P.rowBase + l / SLICE * SLICE) * W;
@@ -430,16 +459,15 @@ bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int wid
             if (l < P.nloc)
                 each(r0 + l, [&](int e, int c) {
                     const size_t at = (size_t)pair_index(sb, W, k, l % SLICE);
-                    R.idx[at] = (uint16_t)(c >= r0 && c < r0 + P.nloc
-                                               ? c - r0
-                                               : P.nlocP + (std::lower_bound(h.begin(), h.end(), c) -
-                                                            h.begin()));
+                    R.idx[at] = (uint16_t)local[c];
                     R.emap[at] = e;
                     ++k;
                 });
             for (; k < W; ++k)
                 R.idx[(size_t)pair_index(sb, W, k, l % SLICE)] = (uint16_t)(P.nlocP + P.nh);
         }
+        for (int l = 0; l < P.nloc; ++l) local[r0 + l] = NONE;
+        for (int h = P.haloBase; h < (int)R.haloSlot.size(); ++h) local[R.haloSlot[h]] = NONE;
     }
     return true;
 }

@@ -86,7 +86,8 @@ int res_reset(const ResPlan* plan, cudaStream_t s);
 bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost& R,
                    int width = 0);
 // The same with consecutive ranges of rowsPerPart rows (whole slices) in the
-// internal order; every row counts as read elsewhere.
-bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int width);
+// internal order; every row counts as read elsewhere.  False also when a part
+// would have more than maxHalo halo values.
+bool res_blocks(int n, const HostLayout& L, int rowsPerPart, ResHost& R, int width, int maxHalo);
 
 }  // namespace cf

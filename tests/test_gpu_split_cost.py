@@ -1,0 +1,87 @@
+"""What the split of a mesh costs the first solves on a topology."""
+import time
+
+import numpy as np
+import pytest
+
+from metal4foam_b200 import _lib, mesh
+
+pytestmark = pytest.mark.gpu
+
+
+def scattered(dims, seed):
+    """An upwind mesh with its cells numbered at random."""
+    s = mesh.upwind3d(dims, seed=seed)
+    p = np.random.default_rng(seed).permutation(s.n)
+    low, upp = s.addr.arrays()[:2]
+    a, b = p[low], p[upp]
+    order = np.lexsort((np.maximum(a, b), np.minimum(a, b)))
+    addr = mesh.ldu_addressing(s.n, np.minimum(a, b)[order].astype(np.int32),
+                               np.maximum(a, b)[order].astype(np.int32))
+    upper = np.where(a > b, s.lower, s.upper)[order]
+    lower = np.where(a > b, s.upper, s.lower)[order]
+    diag, source = np.empty(s.n), np.empty(s.n)
+    diag[p], source[p] = s.diag, s.source
+    return mesh.LduSystem("scattered", addr, diag, upper, lower, source, np.zeros(s.n))
+
+
+def context(s):
+    ctx = _lib.Context(0)
+    ctx.set_topology(s.addr.n, s.addr.nf, *s.addr.arrays())
+    ctx.set_coeffs(s.diag, s.upper, s.lower)
+    return ctx
+
+
+def solve(ctx, s, solver, cluster=0, **kw):
+    x = np.zeros(s.n)
+    l0 = ctx.kernel_launches()
+    t0 = time.perf_counter()
+    ctx.solve(solver, x, s.source, _lib.default_options(clusterMaxCells=cluster, **kw))
+    return x, ctx.kernel_launches() - l0, time.perf_counter() - t0
+
+
+def test_first_solve_on_scattered_cells(require_gpu):
+    """The best first two solves of several fresh contexts, split included,
+    take at most 4 times the best third one (5.2 times when every part sorted
+    and searched its halo)."""
+    s = scattered((23, 23, 23), 1)
+    times = []
+    for _ in range(6):
+        ctx = context(s)
+        times.append([solve(ctx, s, _lib.CF_SOLVER_PBICGSTAB)[2] for _ in range(3)])
+        ctx.close()
+    first, third = min(t[0] + t[1] for t in times), min(t[2] for t in times)
+    assert first < 4.0 * third, (first, third)
+
+
+# the split is made by the first solve, unless it costs more than it gives
+# there: halos of most of the mesh, many cells
+@pytest.mark.parametrize("make,at_once", [
+    (lambda: scattered((13, 13, 12), 2), True),
+    (lambda: scattered((28, 28, 28), 3), False),
+    (lambda: mesh.upwind3d((32, 32, 32), seed=4), True),
+    (lambda: mesh.upwind3d((33, 32, 32), seed=5), False),
+], ids=["scattered_2K", "scattered_22K", "natural_32768", "natural_33792"])
+def test_first_bicgstab_solve_of_a_topology(require_gpu, make, at_once):
+    s = make()
+    ctx = context(s)
+    x1, first, _ = solve(ctx, s, _lib.CF_SOLVER_PBICGSTAB)
+    x2, second, _ = solve(ctx, s, _lib.CF_SOLVER_PBICGSTAB)
+    xg, loop, _ = solve(ctx, s, _lib.CF_SOLVER_PBICGSTAB, -1)
+    assert (first < loop) if at_once else (first == loop), (first, loop)
+    assert second < loop
+    assert np.array_equal(x1, xg) and np.array_equal(x2, xg)
+    ctx.close()
+
+
+# cudaPCG in one cluster: the split of the larger 3-D meshes is made by the
+# third solve; the kernel that runs before has one more launch per restart
+@pytest.mark.parametrize("dims,at_once", [((22, 21, 17), True), ((24, 23, 21), False),
+                                          ((128, 100), True)])
+def test_first_pcg_solve_of_a_small_topology(require_gpu, dims, at_once):
+    s = mesh.varcoeff3d(dims, seed=6, permute=False)
+    ctx = context(s)
+    launches = [solve(ctx, s, _lib.CF_SOLVER_PCG)[1] for _ in range(4)]
+    assert launches[0] == launches[1] and launches[2] == launches[3]
+    assert (launches[2] == launches[0]) if at_once else (launches[2] < launches[0]), launches
+    ctx.close()
