@@ -606,6 +606,11 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
         const int ctas = std::min(CLU_MAX_CTAS, (c->n + CLU_T - 1) / CLU_T);
         if (clu_plan_build(c->n, L, !c->identityPerm, ctas, 0, 0, c->stream, &plan) != CF_OK)
             cudaGetLastError();   // no memory for the split: another path
+        if (plan && plan->split.halo > SPLIT_MAX_HALO)
+        {
+            clu_plan_free(plan);
+            plan = nullptr;
+        }
         c->clu = plan;
     }
     CluPlan* p = static_cast<CluPlan*>(c->clu);

@@ -73,7 +73,7 @@ namespace cf {
 
 struct ResPlan
 {
-    int nparts = 0, W = 0, slots = 0, rowsP = 0, maxLocP = 0, maxHalo = 0;
+    int nparts = 0, W = 0, slots = 0, rowsP = 0, maxHalo = 0;
     int R = 0;                    // rows per thread
     int TB = 0, threads = 0;
     size_t smem = 0;
@@ -733,6 +733,7 @@ int res_plan_build(int device, int n, const HostLayout& L, bool ordered, int npa
     p->W = H.W;
     p->slots = H.slots;
     p->rowsP = H.rowsP;
+    p->maxHalo = H.maxHalo;
     int maxSmem = 0;
     if (cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) !=
         cudaSuccess)
@@ -860,6 +861,11 @@ void resident_build(cf_context* c)
     if (res_plan_build(c->device, c->n, host_layout(c), !c->identityPerm, nparts, 0, 0, c->stream,
                        &p) != CF_OK)
         cudaGetLastError();   // no memory for the split: the graph path
+    if (p && p->maxHalo > SPLIT_MAX_HALO)
+    {
+        res_plan_free(p);
+        p = nullptr;
+    }
     c->resident = p;
 }
 

@@ -79,6 +79,14 @@ int res_launch(const ResPlan* plan, const InnerRun& run, cudaStream_t s);
 // fresh exchange words after a wait has given up
 int res_reset(const ResPlan* plan, cudaStream_t s);
 
+// Halo values of a part from which cudaPCG does not use a split: every part
+// then reads most of the others, and the exchanges cost more than the launches
+// they replace.  Meshes stay far below (2,000 at 900K cells); random links of
+// six per row, ms per solve graph loop / split: 20K in one cluster (6,900 halo
+// values) 0.47 / 0.70, 60K over the SMs (2,300) 0.55 / 0.49, 200K (7,500) 0.77 /
+// 0.89.
+constexpr int SPLIT_MAX_HALO = 4096;
+
 // Splits the rows of L (its internal order; `ordered`: reverse
 // Cuthill-McKee) into nparts parts of equal size (within one row).  Returns
 // false when a part would need more than 65,535 local indices or the rows

@@ -1,4 +1,5 @@
-"""What the split of a mesh costs the first solves on a topology."""
+"""What the split of a mesh costs the first solve that uses it, and meshes
+without locality, which keep the graph loop."""
 import time
 
 import numpy as np
@@ -23,6 +24,19 @@ def scattered(dims, seed):
     diag, source = np.empty(s.n), np.empty(s.n)
     diag[p], source[p] = s.diag, s.source
     return mesh.LduSystem("scattered", addr, diag, upper, lower, source, np.zeros(s.n))
+
+
+def random_links(n, seed):
+    """At most six random neighbours per cell."""
+    rng = np.random.default_rng(seed)
+    a = np.tile(np.arange(n), 3)
+    b = np.concatenate([rng.permutation(n) for _ in range(3)])
+    key = np.unique(np.minimum(a, b)[a != b] * n + np.maximum(a, b)[a != b])
+    low, upp = (key // n).astype(np.int32), (key % n).astype(np.int32)
+    addr = mesh.ldu_addressing(n, low, upp)
+    upper = -rng.uniform(0.5, 2.0, addr.nf)
+    diag = 0.05 - (np.bincount(low, upper, n) + np.bincount(upp, upper, n))
+    return mesh.LduSystem("links", addr, diag, upper, None, rng.standard_normal(n), np.zeros(n))
 
 
 def context(s):
@@ -84,4 +98,18 @@ def test_first_pcg_solve_of_a_small_topology(require_gpu, dims, at_once):
     launches = [solve(ctx, s, _lib.CF_SOLVER_PCG)[1] for _ in range(4)]
     assert launches[0] == launches[1] and launches[2] == launches[3]
     assert (launches[2] == launches[0]) if at_once else (launches[2] < launches[0]), launches
+    ctx.close()
+
+
+# six neighbours per cell at random: a cluster and, at the last size, the split
+# over the SMs would have too many halo values
+@pytest.mark.parametrize("n,whole", [(20000, True), (60000, True), (200000, False)])
+def test_splits_without_locality(require_gpu, n, whole):
+    s = random_links(n, n)
+    ctx = context(s)
+    for _ in range(2):
+        xg, loop, _ = solve(ctx, s, _lib.CF_SOLVER_PCG, -1)
+    x, launches, _ = solve(ctx, s, _lib.CF_SOLVER_PCG)
+    assert (launches < loop) if whole else (launches == loop), (launches, loop)
+    assert np.array_equal(x, xg)
     ctx.close()
