@@ -31,7 +31,7 @@ namespace {
 constexpr int kBlock = 256;
 constexpr int kMaxGroups = 65536;                 // partial sums (one per block)
 constexpr int kTicketSlot = kMaxGroups;           // completion counters live here
-constexpr int kTickets = 64;                      // one 256-byte line of them
+constexpr int kTickets = 32;                      // they take turns; one more for captured calls
 constexpr int kScratchDoubles = kMaxGroups + 32;  // + one 256-byte line for the counter
 
 // The scratch array.  Host code must not pass this name to a kernel: on the
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kBlock)
                            const int* __restrict__ losort, const int* __restrict__ losortStart,
                            const float* __restrict__ x, const float* __restrict__ w,
                            float* __restrict__ y, double* dot, double* scratch,
-                           unsigned int* ticket)
+                           unsigned int* ticket, unsigned int* other)
 {
     __shared__ double sh[kBlock / 32];
     __shared__ bool amLast;
@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(kBlock)
         if (w) acc = (double)wi * (double)sum;
     }
     if (!dot) return;
+    if (other && i == 0) *other = 0u;
     const double part = block_sum(acc, sh);
     if (threadIdx.x == 0)
     {
@@ -274,17 +275,40 @@ extern "C" int cf_ldu_spmv_dot_noalloc(int32_t nCells, const float* diag, const 
     double* scratch = nullptr;
     int rc = scratch_for_current_context(s, &scratch);
     if (rc != CF_OK) return rc;
-    // the completion counter of this call: zero when the library is loaded,
-    // set back to zero by the call's last block.  Calls take turns through the
-    // line's counters, so one whose kernel never ran to its end, or two that
-    // overlap against the contract, do not leave the next call a counter that
-    // is off (a cudaMemsetAsync before every launch did that for 2-3 us)
+    // The completion counter of this call: zero when the library is loaded,
+    // set back to zero by the call's last block.  Two calls that overlap
+    // against the contract can leave theirs off, so calls take turns through
+    // the counters, and each also clears the one half a round ahead: whatever
+    // a counter holds, it is zero when its turn comes (a cudaMemsetAsync before
+    // every launch did that for 2-3 us).  A captured call has one counter for
+    // every replay and no say in what runs between them: it keeps the memset,
+    // as a node of the graph, and a counter of its own.
     static std::atomic<unsigned int> turn{0};
-    unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch + kTicketSlot) +
-                           turn.fetch_add(1, std::memory_order_relaxed) % kTickets;
+    unsigned int* const tickets = reinterpret_cast<unsigned int*>(scratch + kTicketSlot);
+    unsigned int* ticket = nullptr;
+    unsigned int* other = nullptr;
+    if (dot)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cudaGetLastError();
+        if (cs == cudaStreamCaptureStatusActive)
+        {
+            ticket = tickets + kTickets;
+            const cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s);
+            if (e != cudaSuccess)
+                return cf::fail(CF_ERR_CUDA,
+                                std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+        }
+        else
+        {
+            const unsigned int k = turn.fetch_add(1, std::memory_order_relaxed);
+            ticket = tickets + k % kTickets;
+            other = tickets + (k + kTickets / 2) % kTickets;
+        }
+    }
     k_ldu_spmv_dot_noalloc<<<(unsigned)groups, kBlock, 0, s>>>(
         nCells, diag, upper, lower, lowAddr, uppAddr, ownStartAddr, losortAddr, losortStartAddr, x,
-        w, y, dot, scratch, ticket);
+        w, y, dot, scratch, ticket, other);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return cf::fail(CF_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
