@@ -137,7 +137,10 @@ typedef struct
                                   cluster, larger ones up to 6144 cells per
                                   SM (about 900,000) as one cooperative
                                   launch.  GAMG: the levels of at most 4096
-                                  cells in one cluster.  < 0: the graph loop
+                                  cells in one cluster.  > 0: the same for
+                                  meshes (batches: with every system, GAMG:
+                                  with the finest level of the cluster) of at
+                                  most this many cells.  < 0: the graph loop
                                   always, launches for every level         */
     int32_t preconditioner;    /* cudaPCG: CF_PRECOND_CHEBYSHEV (default) or
                                   CF_PRECOND_GAMG: z = M r is one symmetric

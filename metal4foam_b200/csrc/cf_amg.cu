@@ -1093,6 +1093,12 @@ void amg_release(cf_context* c)
     c->amg = nullptr;
 }
 
+int amg_cluster_cells(const cf_context* c)
+{
+    const AmgData* d = static_cast<const AmgData*>(c->amg);
+    return d && d->tailFrom ? d->lv[d->tailFrom].n : 0;
+}
+
 int amg_levels(const cf_context* c)
 {
     const AmgData* d = static_cast<const AmgData*>(c->amg);

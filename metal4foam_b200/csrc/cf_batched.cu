@@ -1634,6 +1634,8 @@ int batch_solve(cf_batch* bt, double* const* psi, const double* const* src, bool
                                                     o->chebyshevRatio, bt->d_chebC);
         CFB_LAUNCH();
     }
+    int maxCells = 0;   // of a system
+    for (const auto& y : bt->sys) maxCells = std::max(maxCells, (int)y.n);
     int outer = 0;
     bool all_done = false;
     for (outer = 0; outer <= o->maxRestarts; ++outer)
@@ -1646,8 +1648,8 @@ int batch_solve(cf_batch* bt, double* const* psi, const double* const* src, bool
         kb_mean<1><<<tgrid(bt, (const void*)kb_mean<1>), NT, 0, s>>>(B);
         CFB_LAUNCH();
         bool whole = false;
-        if (bt->whole && o->graph && o->persistentMaxCells <= 0 && o->clusterMaxCells >= 0 &&
-            o->maxIter > 0)
+        if (bt->whole && o->graph && o->persistentMaxCells <= 0 &&
+            cluster_allows(o->clusterMaxCells, maxCells) && o->maxIter > 0)
             CFB_TRY(whole_loop(bt, o, &whole));
         if (!whole)
         {

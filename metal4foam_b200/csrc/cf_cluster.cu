@@ -346,7 +346,7 @@ int cluster_shift(int n)
     return shift;
 }
 
-int cluster_inner(cf_context* c, int order, int maxCells, bool* ran)
+int cluster_inner(cf_context* c, int order, bool* ran)
 {
     *ran = false;
     // one row per thread (at most 16 x 1024 rows) and columns mostly in the

@@ -264,10 +264,16 @@ int launch_spmv32_v(cf_context* c, const float* diag, const float* x, const floa
 // *ran tells whether it was launched.  persistent_status reads the grid
 // barrier's error word after the stream has completed.
 int persistent_inner(cf_context* c, int kind, int order, int maxCells, bool* ran);
+// cf_options::clusterMaxCells: may a mesh (or a GAMG level) of n cells run in a
+// cluster, or as one launch?
+inline bool cluster_allows(int maxCells, int n)
+{
+    return maxCells == 0 || (maxCells > 0 && n <= maxCells);
+}
+
 // Inner PCG inside one thread-block cluster (cf_cluster.cu) for meshes of
-// at most min(maxCells, 16384) cells whose columns lie mostly in their own
-// CTA; *ran tells whether it was launched.
-int cluster_inner(cf_context* c, int order, int maxCells, bool* ran);
+// at most 16384 cells whose columns lie mostly in their own CTA; *ran tells whether it was launched.
+int cluster_inner(cf_context* c, int order, bool* ran);
 // The same for meshes with at most six neighbours per cell and up to
 // CLU_MAX_ROWS cells, matrix and vectors in registers (cf_clupcg.cu); runs
 // and completes the inner solve as resident_inner does.
@@ -342,6 +348,8 @@ int amg_prepare(cf_context* c, int coarsestCap, bool profile = false);
 int amg_stage(cf_context* c, int deflate, float scaleCorrection);
 int launch_amg_body(cf_context* c, int degree, cudaGraphConditionalHandle h, int useCond,
                     int* kernels);
+// cells of the finest level that runs in the cluster (0: none)
+int amg_cluster_cells(const cf_context* c);
 int amg_levels(const cf_context* c);
 int amg_level_cells(const cf_context* c, int level);
 void amg_release(cf_context* c);

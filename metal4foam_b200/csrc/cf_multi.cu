@@ -1021,7 +1021,7 @@ int solve_multi_streams(cf_context* c, int32_t solver, int32_t nrhs, double* psi
     std::vector<std::string> msg(nrhs);
     // Meshes that run as one CTA per SM: up to three components in one launch
     // (cf_resbicg.cu; 36^3 7.1 -> 5.3 ms, 64^3 19.5 -> 15.1, 72^3 22.1 -> 18.0).
-    ResBicgTeam* const team = o->graph && o->clusterMaxCells >= 0 && nrhs == W
+    ResBicgTeam* const team = o->graph && cluster_allows(o->clusterMaxCells, c->n) && nrhs == W
                                   ? res_bicg_team(c, W) : nullptr;
     // (without a team concurrent graph loops: taking turns on all SMs one
     // component at a time is slower, 64^3 with three 22.0 ms against 19.9)

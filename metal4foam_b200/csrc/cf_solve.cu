@@ -245,7 +245,8 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     };
     // the whole inner solve as one launch, in one cluster or on the mesh's
     // split over the SMs
-    if (kind == 1 && useGraph && clusterMax >= 0 && spmv_default(c) && !mean)
+    const bool oneLaunch = useGraph && spmv_default(c) && cluster_allows(clusterMax, c->n);
+    if (kind == 1 && oneLaunch && !mean)
     {
         bool whole = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
@@ -254,8 +255,7 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
         c->pendingBodyKernels = 0;
         if (whole) return finish();
     }
-    if (kind == 0 && useGraph && clusterMax >= 0 && persistMax <= 0 && spmv_default(c) &&
-        !c->amgActive)
+    if (kind == 0 && oneLaunch && persistMax <= 0 && !c->amgActive)
     {
         bool resident = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
@@ -303,8 +303,8 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     if (maxIter > 0)
     {
         // small PCG systems: the whole loop inside one thread-block cluster
-        if (useGraph && spmv_default(c) && kind == 0 && clusterMax >= 0 && !c->amgActive)
-            CF_TRY(cluster_inner(c, order, clusterMax == 0 ? 16384 : clusterMax, &clustered));
+        if (oneLaunch && kind == 0 && !c->amgActive)
+            CF_TRY(cluster_inner(c, order, &clustered));
         // opt-in: the whole loop as one cooperative kernel
         if (!clustered && useGraph && spmv_default(c) && !c->amgActive)
             CF_TRY(persistent_inner(c, kind, kind == 0 ? order : 1, persistMax, &persistent));
@@ -467,7 +467,7 @@ int solve_device(cf_context* c, int solver, double* psi_dev, const double* src_d
             CF_TRY(amg_prepare(c, o->nCellsInCoarsestLevel, o->profile != 0));
             CF_TRY(amg_stage(c, deflate ? 1 : 0, (float)o->scaleCorrection));
             c->amgActive = true;
-            c->amgLaunches = o->clusterMaxCells < 0;
+            c->amgLaunches = !cluster_allows(o->clusterMaxCells, amg_cluster_cells(c));
         }
 
         // Chebyshev setup (metalFoamSolver.C:224-249); with GAMG the
