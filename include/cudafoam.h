@@ -220,7 +220,9 @@ int cf_context_set_stream(cf_context* ctx, void* stream);
 int cf_context_set_reorder(cf_context* ctx, int32_t mode);
 /* Polls a bounded device-side wait of this context makes before it gives
  * up, which ends the kernel.  A resident inner solve (clusterMaxCells) then
- * runs through the graph loop instead; with the grid barriers of persistent
+ * runs through the graph loop instead, and so do the next ones: two, and
+ * twice as many after each further time in a row, until a call of this
+ * function or a new topology; with the grid barriers of persistent
  * inner solves (persistentMaxCells) the solve returns
  * CF_ERR_DEVICE_TIMEOUT, leaving the context usable.  0 restores the
  * default, 2^24 polls of about 64 ns each.  No reference counterpart. */

@@ -1052,6 +1052,7 @@ struct cf_batch
         CluSys* d_list = nullptr;
     };
     bool whole = false;
+    WholeBackoff backoff;
     int wholeOrder = -1;                   // chebyshevOrder of the uploaded lists
     std::vector<CluPlan*> clu;
     std::vector<ResPlan*> res;
@@ -1524,6 +1525,7 @@ int whole_build(cf_batch* bt, int reorder)
 int whole_loop(cf_batch* bt, const cf_options* o, bool* ran)
 {
     *ran = false;
+    if (!bt->backoff.may()) return CF_OK;
     cudaStream_t s = bt->stream;
     std::unique_lock<std::mutex> turn(res_device_lock(bt->device), std::defer_lock);
     if (!bt->slots.empty()) turn.lock();
@@ -1578,9 +1580,11 @@ int whole_loop(cf_batch* bt, const cf_options* o, bool* ran)
     for (int i = 0; i < bt->S; ++i) gaveUp = gaveUp || bt->h_st[i].waitErr;
     if (!gaveUp)
     {
+        bt->backoff.worked();
         *ran = true;
         return CF_OK;
     }
+    bt->backoff.gaveUp();
     for (const ResPlan* p : bt->res)
         if (p) CFB_TRY(res_reset(p, s));
     for (int i = 0; i < bt->S; ++i)

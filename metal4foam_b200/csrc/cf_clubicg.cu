@@ -477,8 +477,10 @@ int clu_bicg_inner(cf_context* c, double target, int maxIter, int ips, int stagL
     {
         // a wait gave up: this solve goes through the graph path
         CLB_CUDA(cudaMemsetAsync(&c->d_st->waitErr, 0, sizeof(int), s));
+        c->backoff.gaveUp();
         return CF_OK;
     }
+    c->backoff.worked();
     *ran = true;
     return CF_OK;
 }

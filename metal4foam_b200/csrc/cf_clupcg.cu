@@ -630,8 +630,10 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
     {
         // a wait gave up: this solve goes through the graph path
         CLU_CUDA(cudaMemsetAsync(&c->d_st->waitErr, 0, sizeof(int), s));
+        c->backoff.gaveUp();
         return CF_OK;
     }
+    c->backoff.worked();
     *ran = true;
     return CF_OK;
 }

@@ -93,6 +93,7 @@ void free_topology(cf_context* c)
     clu_bicg_release(c);
     res_bicg_release(c);
     c->solves = c->bicgSolves = 0;
+    c->backoff = WholeBackoff();
     c->hostCol.clear();
     c->hostSliceOff.clear();
     for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
@@ -575,6 +576,7 @@ extern "C" int cf_context_set_wait_limit(cf_context* c, int64_t polls)
 {
     if (!c || polls < 0) return fail(CF_ERR_INVALID_ARG, "bad wait limit");
     c->waitPolls = polls == 0 ? (1LL << 24) : (long long)polls;
+    c->backoff = WholeBackoff();
     return CF_OK;
 }
 
@@ -904,6 +906,7 @@ int context_clone_sync(cf_context* src, cf_context* c)
     c->val32Sym = src->val32Sym;
     c->transposed = src->transposed;
     c->waitPolls = src->waitPolls;
+    c->backoff = src->backoff;
     c->cluBicg = src->cluBicg;   // (made before: clu_bicg_prepare)
     c->cluBicgTried = true;
     c->cluBicgShared = true;

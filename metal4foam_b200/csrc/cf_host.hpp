@@ -21,6 +21,33 @@ namespace cf {
 struct ResBicgTeam;
 }
 
+namespace cf {
+
+// After a wait of a whole inner solve (cf_clupcg.cu, cf_resident.cu, ...) has
+// run out, because something else on the GPU keeps some of its CTAs off the
+// SMs, the next 2 inner solves go through the graph loop, after every further
+// time twice as many: a wait takes seconds to run out.
+struct WholeBackoff
+{
+    int times = 0;   // in a row
+    int skip = 0;    // inner solves still to go through the graph loop
+
+    bool may()
+    {
+        if (skip == 0) return true;
+        --skip;
+        return false;
+    }
+    void gaveUp()
+    {
+        times = std::min(times + 1, 10);
+        skip = 1 << times;
+    }
+    void worked() { times = 0; }
+};
+
+}  // namespace cf
+
 struct cf_context
 {
     // device / runtime (metalFoamBackend::Impl::init, metalFoamBackend.C:192-282)
@@ -135,6 +162,7 @@ struct cf_context
     cf::ResBicgTeam* resBicgTeam = nullptr; // clones that run their inner solves together
     int solves = 0;                        // cudaPCG solves on this topology so far
     int bicgSolves = 0;                    // cudaPBiCGStab solves on it
+    cf::WholeBackoff backoff;              // of whole inner solves
     int concurrent = 1;                    // solves that cf_solve_many_device runs side by side
     std::vector<int32_t> hostCol;          // host copy of the columns, kept for the splits
     std::vector<int32_t> hostSliceOff;

@@ -1072,6 +1072,10 @@ int solve_multi_streams(cf_context* c, int32_t solver, int32_t nrhs, double* psi
     for (int w : inlineRuns) run(w, nullptr);
     for (auto& t : pool) t.join();
     if (team) res_bicg_team_free(team);
+    // (the next solve's components start from the one that gave up most)
+    c->backoff = c->clones[0]->backoff;
+    for (int w = 1; w < W; ++w)
+        if (c->clones[w]->backoff.times > c->backoff.times) c->backoff = c->clones[w]->backoff;
     for (int k = 0; k < nrhs; ++k)
         if (rc[k] != CF_OK) return fail(rc[k], "component " + std::to_string(k) + ": " + msg[k]);
     for (int w = 0; w < W; ++w)

@@ -740,8 +740,10 @@ int launch(cf_context* const* ctx, const InnerRun* runs, int count, bool* ran)
         RSB_CUDA(cudaMemsetAsync(w->base, 0, w->bytes, s));
         RSB_CUDA(cudaMemsetAsync(&c->d_st->waitErr, 0, sizeof(int), s));
         RSB_CUDA(cudaStreamSynchronize(s));
+        for (int k = 0; k < count; ++k) ctx[k]->backoff.gaveUp();
         return CF_OK;
     }
+    for (int k = 0; k < count; ++k) ctx[k]->backoff.worked();
     *ran = true;
     return CF_OK;
 }

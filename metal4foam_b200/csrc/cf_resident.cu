@@ -903,8 +903,10 @@ int resident_inner(cf_context* c, const double* mean, double target, int maxIter
         const int rr = res_reset(p, s);
         if (rr != CF_OK) return rr;
         RES_CUDA(cudaMemsetAsync(&c->d_st->waitErr, 0, sizeof(int), s));
+        c->backoff.gaveUp();
         return CF_OK;
     }
+    c->backoff.worked();
     *ran = true;
     return CF_OK;
 }

@@ -244,18 +244,22 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
         return CF_OK;
     };
     // the whole inner solve as one launch, in one cluster or on the mesh's
-    // split over the SMs
+    // split over the SMs, unless its waits have run out lately
+    bool loopOnly = false;
     const bool oneLaunch = useGraph && spmv_default(c) && cluster_allows(clusterMax, c->n);
-    if (kind == 1 && oneLaunch && !mean)
+    if (kind == 1 && oneLaunch && !mean && c->backoff.may())
     {
         bool whole = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
         CF_TRY(clu_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
-        if (!whole) CF_TRY(res_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
+        if (!whole && !c->backoff.skip)
+            CF_TRY(res_bicg_inner(c, target, maxIter, ips, stagLimit, &whole));
         c->pendingBodyKernels = 0;
         if (whole) return finish();
     }
     if (kind == 0 && oneLaunch && persistMax <= 0 && !c->amgActive)
+        loopOnly = !c->backoff.may();
+    if (kind == 0 && oneLaunch && persistMax <= 0 && !c->amgActive && !loopOnly)
     {
         bool resident = false;
         CF_CUDA(cudaEventRecord(c->ev0, s));
@@ -270,10 +274,11 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
                           : c->n <= CLU_MAX_ROWS && later &&
                                 c->n >= RESIDENT_MIN_ROWS_PER_SM * c->numSMs && c->maxRowLen >= 4)
             CF_TRY(clu_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
-        if (!resident)
+        if (!resident && !c->backoff.skip)
             CF_TRY(resident_inner(c, mean, target, maxIter, ips, order, stagLimit, &resident));
         c->pendingBodyKernels = 0;
         if (resident) return finish();
+        loopOnly = c->backoff.skip > 0;
     }
     k_inner_setup<<<1, 32, 0, s>>>(c->d_st, target, maxIter, ips, stagLimit);
     CF_LAUNCH();
@@ -303,7 +308,7 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     if (maxIter > 0)
     {
         // small PCG systems: the whole loop inside one thread-block cluster
-        if (oneLaunch && kind == 0 && !c->amgActive)
+        if (oneLaunch && kind == 0 && !c->amgActive && !loopOnly)
             CF_TRY(cluster_inner(c, order, &clustered));
         // opt-in: the whole loop as one cooperative kernel
         if (!clustered && useGraph && spmv_default(c) && !c->amgActive)
