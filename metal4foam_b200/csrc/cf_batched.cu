@@ -1331,6 +1331,8 @@ int persistent_loop(cf_batch* bt, int order, bool* ran)
     GridBar bar{bt->d_bar, bt->d_bar + 1, reinterpret_cast<int*>(bt->d_bar + 2), 1ull << 24};
     int ord = order;
     void* args[] = {(void*)&B, (void*)&ord, (void*)&bar};
+    // (until the launch has ended: its grid barriers need all blocks on the device)
+    std::lock_guard<std::mutex> turn(res_device_lock(bt->device));
     const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(NT), args, 0, s);
     if (e != cudaSuccess)
         return fail(CF_ERR_CUDA, std::string("cudaLaunchCooperativeKernel: ") + cudaGetErrorString(e));

@@ -287,11 +287,12 @@ int launch_bicg_cd_v(cf_context* c, const BicgBufs& B, cudaGraphConditionalHandl
 int launch_spmv32_v(cf_context* c, const float* diag, const float* x, const float* w, float* y,
                     double* out);
 
-// Inner solve as one cooperative kernel (cf_persist.cu) when the mesh has
+// Inner PCG as one cooperative kernel (cf_persist.cu) when the mesh has
 // at most maxCells cells (<= 0: never) and the launch fits;
 // *ran tells whether it was launched.  persistent_status reads the grid
-// barrier's error word after the stream has completed.
-int persistent_inner(cf_context* c, int kind, int order, int maxCells, bool* ran);
+// barrier's error word after the stream has completed.  The caller holds the
+// device's lock (res_device_lock) until then.
+int persistent_inner(cf_context* c, int order, int maxCells, bool* ran);
 // cf_options::clusterMaxCells: may a mesh (or a GAMG level) of n cells run in a
 // cluster, or as one launch?
 inline bool cluster_allows(int maxCells, int n)

@@ -185,10 +185,10 @@ __global__ void __launch_bounds__(NT) kp_pcg(DevSell A, PcgBufs B, int order, In
 
 namespace cf {
 
-int persistent_inner(cf_context* c, int kind, int order, int maxCells, bool* ran)
+int persistent_inner(cf_context* c, int order, int maxCells, bool* ran)
 {
     *ran = false;
-    if (kind != 0 || maxCells <= 0 || c->n > maxCells || !c->coopLaunch || !c->d_bar)
+    if (maxCells <= 0 || c->n > maxCells || !c->coopLaunch || !c->d_bar)
         return CF_OK;
     const int n = c->n;
     const int need = (n + NT - 1) / NT;

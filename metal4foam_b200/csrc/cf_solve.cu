@@ -2,11 +2,13 @@
 // refinement driver, and the operator entry points of the C ABI.
 #include "cudafoam.h"
 #include "cf_host.hpp"
+#include "cf_resident.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -305,14 +307,21 @@ int inner_solve(cf_context* c, int kind, const double* mean, double target, int 
     CF_CUDA(cudaEventRecord(c->ev0, s));
     bool persistent = false;
     bool clustered = false;
+    std::unique_lock<std::mutex> turn;
     if (maxIter > 0)
     {
         // small PCG systems: the whole loop inside one thread-block cluster
         if (oneLaunch && kind == 0 && !c->amgActive && !loopOnly)
             CF_TRY(cluster_inner(c, order, &clustered));
         // opt-in: the whole loop as one cooperative kernel
-        if (!clustered && useGraph && spmv_default(c) && !c->amgActive)
-            CF_TRY(persistent_inner(c, kind, kind == 0 ? order : 1, persistMax, &persistent));
+        if (!clustered && useGraph && spmv_default(c) && kind == 0 && !c->amgActive &&
+            persistMax > 0 && c->n <= persistMax)
+        {
+            // (its grid barriers need all blocks on the device: until it has ended)
+            turn = std::unique_lock<std::mutex>(res_device_lock(c->device));
+            CF_TRY(persistent_inner(c, order, persistMax, &persistent));
+            if (!persistent) turn.unlock();
+        }
         if (persistent || clustered)
         {
             c->pendingBodyKernels = 0;

@@ -168,3 +168,47 @@ def test_many_bicgstab_forms(require_gpu, rows, count, form):
         assert (a < b) if form == "whole" else (a == b), (a, b)
     for c in ctxs:
         c.close()
+
+
+def test_persistent_launches_take_turns(require_gpu):
+    """The opt-in persistent inner solves, of a context and of a batch, at the
+    same time as solves on the split over the SMs: none runs into its wait
+    limit, all results as alone."""
+    ss = [mesh.varcoeff3d((40, 40, 22), seed=50, permute=True),
+          mesh.varcoeff3d((44, 42, 40), seed=51, permute=True)]
+    ctxs = [context(s) for s in ss]
+    bs = [mesh.poisson2d(100, 90, seed=52), mesh.varcoeff3d((24, 24, 24), seed=53)]
+    bt = batch(bs)
+
+    def opts(persistent):
+        return _lib.default_options(persistentMaxCells=1000000 if persistent else 0, maxIter=200)
+
+    def one(k):
+        if k < 2:
+            x = np.zeros(ss[k].n)
+            ctxs[k].solve(_lib.CF_SOLVER_PCG, x, ss[k].source, opts(k == 0))
+            return [x]
+        xs = [np.zeros(s.n) for s in bs]
+        bt.solve(xs, [s.source for s in bs], opts(True))
+        return xs
+
+    for _ in range(3):
+        alone = [one(k) for k in range(3)]
+    out = [[] for _ in range(3)]
+
+    def work(k):
+        for _ in range(8):
+            out[k].append(one(k))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(3):
+        assert len(out[k]) == 8
+        for xs in out[k]:
+            assert all(np.array_equal(x, a) for x, a in zip(xs, alone[k])), k
+    for c in ctxs:
+        c.close()
+    bt.close()
