@@ -489,9 +489,11 @@ int clu_plan_upload(ResHost& H, int ctas, int buffers, int nd, long long entOff,
         for (int32_t& r : H.rowMap)
             if (r >= 0) r += rowOff;
         p = new CluPlan();
+        p->allocs.reserve(1);
     }
     catch (...)
     {
+        clu_plan_free(p);
         return CF_OK;   // no memory for the split
     }
     p->W = W;
@@ -601,11 +603,18 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
     {
         c->cluTried = true;
         if (c->hostSliceOff.empty()) return CF_OK;
-        const HostLayout L = host_layout(c);
         CluPlan* plan = nullptr;
         const int ctas = std::min(CLU_MAX_CTAS, (c->n + CLU_T - 1) / CLU_T);
-        if (clu_plan_build(c->n, L, !c->identityPerm, ctas, 0, 0, c->stream, &plan) != CF_OK)
-            cudaGetLastError();   // no memory for the split: another path
+        try
+        {
+            if (clu_plan_build(c->n, host_layout(c), !c->identityPerm, ctas, 0, 0, c->stream,
+                               &plan) != CF_OK)
+                cudaGetLastError();   // no memory for the split: another path
+        }
+        catch (...)
+        {
+            return CF_OK;             // (for the host's copy of the layout)
+        }
         if (plan && plan->split.halo > SPLIT_MAX_HALO)
         {
             clu_plan_free(plan);

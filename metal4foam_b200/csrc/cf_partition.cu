@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <new>
 #include <numeric>
 #include <thread>
 #include <vector>
@@ -99,7 +100,8 @@ void csr_of_layout(int n, const HostLayout& L, int threads, Csr& g)
 }
 
 // rows of it[lo, hi) into parts p0 .. p0 + np - 1: part[row]
-// (the two halves on two threads while `threads` > 1)
+// (the two halves on two threads while `threads` > 1).  Out of memory on either
+// of them throws here, once the other has ended.
 void bisect(std::vector<Item>& it, int lo, int hi, int p0, int np, std::vector<int32_t>& part,
             std::vector<Item>& tmp, int threads)
 {
@@ -167,14 +169,30 @@ void bisect(std::vector<Item>& it, int lo, int hi, int p0, int np, std::vector<i
         a = i0;
         b = i0 + neq;
     }
-    std::thread left;
+    struct Half
+    {
+        std::thread thread;
+        bool failed = false;
+        void join()
+        {
+            if (thread.joinable()) thread.join();
+        }
+        ~Half() { join(); }
+    } left;
     bool started = false;
     if (threads > 1)
     {
         try
         {
-            left = std::thread([&, lo, cut, p0, pl, threads]() {
-                bisect(it, lo, cut, p0, pl, part, tmp, threads / 2);
+            left.thread = std::thread([&, lo, cut, p0, pl, threads]() {
+                try
+                {
+                    bisect(it, lo, cut, p0, pl, part, tmp, threads / 2);
+                }
+                catch (...)
+                {
+                    left.failed = true;
+                }
             });
             started = true;
         }
@@ -184,7 +202,8 @@ void bisect(std::vector<Item>& it, int lo, int hi, int p0, int np, std::vector<i
     }
     if (!started) bisect(it, lo, cut, p0, pl, part, tmp, 1);
     bisect(it, cut, hi, p0 + pl, np - pl, part, tmp, started ? threads - threads / 2 : 1);
-    if (started) left.join();
+    left.join();
+    if (left.failed) throw std::bad_alloc();
 }
 
 }  // namespace

@@ -724,9 +724,11 @@ int res_plan_build(int device, int n, const HostLayout& L, bool ordered, int npa
             for (int32_t& r : H.rowMap)
                 if (r >= 0) r += rowOff;
         p = new ResPlan();
+        p->allocs.reserve(16);
     }
     catch (...)
     {
+        res_plan_free(p);
         return CF_OK;   // no memory for the split
     }
     p->nparts = nparts;
@@ -858,9 +860,16 @@ void resident_build(cf_context* c)
     const int nparts = std::min(c->numSMs, RES_MAX_PARTS);
     if (!c->coopLaunch || c->n > (long long)nparts * RES_MAX_ROWS || c->hostSliceOff.empty()) return;
     ResPlan* p = nullptr;
-    if (res_plan_build(c->device, c->n, host_layout(c), !c->identityPerm, nparts, 0, 0, c->stream,
-                       &p) != CF_OK)
-        cudaGetLastError();   // no memory for the split: the graph path
+    try
+    {
+        if (res_plan_build(c->device, c->n, host_layout(c), !c->identityPerm, nparts, 0, 0,
+                           c->stream, &p) != CF_OK)
+            cudaGetLastError();   // no memory for the split: the graph path
+    }
+    catch (...)
+    {
+        return;                   // (for the host's copy of the layout)
+    }
     if (p && p->maxHalo > SPLIT_MAX_HALO)
     {
         res_plan_free(p);
