@@ -327,7 +327,9 @@ int cf_solve_adjoint_device(cf_context* ctx, int32_t solver, const double* x,
  * decisions, same stopping tests as cf_solve on each system alone): every
  * phase of the iteration is one launch over all still-active systems and
  * the iterations run in a device-side CUDA-graph loop until the last
- * system has finished. */
+ * system has finished; a batch without solo systems (below) runs every
+ * inner solve whole where all of them fit on chip (clusterMaxCells).  The
+ * forms add their FP64 sums in orders of their own, as cf_solve's do. */
 typedef struct cf_batch cf_batch;
 
 int cf_batch_create(cf_batch** out, int32_t device);
@@ -658,7 +660,7 @@ int cf_subdomain_set_coeffs(cf_subdomain* sub, const double* diag, const double*
  * halos exchanged before each SpMV; preconditioner Chebyshev-Jacobi; one
  * host synchronisation per inner iteration); psi (in/out) and source are
  * this subdomain's host arrays.  With no interfaces and one subdomain the
- * result equals cf_solve's bit for bit. */
+ * result equals cf_solve's with clusterMaxCells < 0 bit for bit. */
 int cf_subdomain_solve(cf_subdomain* sub, int32_t solver, double* psi, const double* source,
                        const cf_options* opts, const cf_comm* comm, cf_performance* perf);
 

@@ -16,7 +16,8 @@
 // the last tile of a system to finish (per-system atomic ticket) folds the
 // system's partials in tile order and updates that system's scalars.
 // Per row the arithmetic is the single-system kernels' (same row functions),
-// so every system follows exactly the iteration it would follow alone.
+// so every system follows the iteration it would follow alone, up to the order
+// in which the FP64 sums are added.
 #include "cudafoam.h"
 #include "cf_cluster_ll.cuh"
 #include "cf_host.hpp"

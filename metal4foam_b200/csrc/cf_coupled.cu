@@ -27,7 +27,7 @@
 // (gathered into a send buffer, then cf_comm.exchange).  Every kernel runs
 // on the grid of its single-domain counterpart with the same per-row
 // arithmetic, so a subdomain without interfaces whose communication is the
-// identity returns bit for bit what cf_solve returns.  Decisions depend
+// identity returns bit for bit what cf_solve's graph loop returns.  Decisions depend
 // only on globally reduced values, so every subdomain takes the same steps
 // (the same collectives in the same order).  One host synchronisation per
 // inner iteration reads the stopping state.

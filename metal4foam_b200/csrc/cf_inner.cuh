@@ -1,6 +1,6 @@
-// cf_inner.cuh -- what the kernels that run a whole inner PCG share
-// (cf_resident.cu, cf_cluster.cu): the solver state every CTA keeps, and a
-// row of A x with its entries in registers.
+// cf_inner.cuh -- what the kernels that run a whole inner solve share
+// (cf_clupcg.cu, cf_resident.cu, cf_clubicg.cu, cf_resbicg.cu): the solver state
+// every CTA keeps, and a row of A x with its entries in registers.
 #pragma once
 
 #include <cuda_runtime.h>

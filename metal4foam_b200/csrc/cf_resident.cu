@@ -98,7 +98,7 @@ constexpr int RES_MAX_ROWS = 6144;   // rows of a part at most (the last entry o
 constexpr int RES_COPIES = 8;        // copies of every reduction word
 // A part's words have a 128-byte line of their own (with four parts to a line,
 // whose writers and pollers meet in L2: 64^3 Jacobi 8.66 us per iteration, 8.29
-// so; prism 200K order 8 18.1 and 17.6).
+// so; prism 200K order 8 18.1 and 17.9).
 constexpr int RES_STRIDE = 16;       // 8-byte words
 constexpr size_t RES_RED_WORDS = (size_t)RES_COPIES * RES_MAX_PARTS * RES_STRIDE;
 constexpr int RES_HQ = 4;            // halo slots a thread keeps in registers
