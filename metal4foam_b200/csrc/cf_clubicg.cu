@@ -436,7 +436,8 @@ void clu_bicg_prepare(cf_context* c, bool first)
     ResHost H;
     try
     {
-        if (!res_blocks(c->n, host_layout(c), per * NT, H, 4,
+        const LentLayout lent(c);
+        if (!res_blocks(c->n, lent.L, per * NT, H, 4,
                         first ? CLB_FIRST_HALO : CLU_MAX_HALO))
         {
             c->cluBicgTried = !first;

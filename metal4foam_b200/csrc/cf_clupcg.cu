@@ -605,15 +605,11 @@ int clu_inner(cf_context* c, const double* mean, double target, int maxIter, int
         if (c->hostSliceOff.empty()) return CF_OK;
         CluPlan* plan = nullptr;
         const int ctas = std::min(CLU_MAX_CTAS, (c->n + CLU_T - 1) / CLU_T);
-        try
         {
-            if (clu_plan_build(c->n, host_layout(c), !c->identityPerm, ctas, 0, 0, c->stream,
-                               &plan) != CF_OK)
+            const LentLayout lent(c);
+            if (clu_plan_build(c->n, lent.L, !c->identityPerm, ctas, 0, 0, c->stream, &plan) !=
+                CF_OK)
                 cudaGetLastError();   // no memory for the split: another path
-        }
-        catch (...)
-        {
-            return CF_OK;             // (for the host's copy of the layout)
         }
         if (plan && plan->split.halo > SPLIT_MAX_HALO)
         {

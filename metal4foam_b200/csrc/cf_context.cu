@@ -251,15 +251,19 @@ int check_addressing(int32_t n, int32_t nf, const int32_t* low, const int32_t* u
     return validate_addressing(n, nf, low, upp, own, los, losS);
 }
 
-HostLayout host_layout(const cf_context* c)
+LentLayout::LentLayout(cf_context* ctx) : c(ctx)
 {
-    HostLayout L;
-    L.col = c->hostCol;
-    L.sliceOff = c->hostSliceOff;
+    L.col.swap(c->hostCol);
+    L.sliceOff.swap(c->hostSliceOff);
     L.nslices = c->nslices;
     L.nnzp = c->nnzp;
     L.maxw = c->maxRowLen;
-    return L;
+}
+
+LentLayout::~LentLayout()
+{
+    L.col.swap(c->hostCol);
+    L.sliceOff.swap(c->hostSliceOff);
 }
 
 // Internal ordering + SELL-32 layout of one mesh on the host.

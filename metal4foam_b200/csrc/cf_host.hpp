@@ -330,8 +330,17 @@ void res_bicg_team_free(ResBicgTeam* t);
 // log2(rows per CTA) of the cluster PCG for an n-row mesh: the smallest
 // power of two >= 32 that needs at most 16 CTAs.
 int cluster_shift(int n);
-// The host layout a split needs, from the copies the context keeps.
-HostLayout host_layout(const cf_context* c);
+// The host layout a split needs: the arrays the context keeps, lent while this
+// lives.
+struct LentLayout
+{
+    cf_context* c;
+    HostLayout L;
+    explicit LentLayout(cf_context* ctx);
+    ~LentLayout();
+    LentLayout(const LentLayout&) = delete;
+    LentLayout& operator=(const LentLayout&) = delete;
+};
 int persistent_status(cf_context* c);
 
 // Inner PCG as one launch with the mesh split over the SMs (cf_resident.cu),

@@ -149,9 +149,7 @@ void bisect(std::vector<Item>& it, int lo, int hi, int p0, int np, std::vector<i
         const int val = below == cut ? base + v + 1 : base + v;
         // stable three-way split: c < val, c == val, c > val
         int i0 = a;
-        int neq = 0;
-        for (int i = a; i < b; ++i)
-            if (it[i].c[k] == val) ++neq;
+        const int neq = hist[val - base + 1];
         std::vector<Item>& t = tmp;
         int eq = 0, gt = neq;
         for (int i = a; i < b; ++i)
@@ -268,10 +266,28 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
                     break;
                 }
     });
-    for (int r = 0; r < n; ++r)
+    // rows of every part in each of `nt` ranges of rows: inner, boundary; then,
+    // summed up, the local index of the next one there
+    std::vector<std::vector<int32_t>> next(nt);
+    for (auto& v : next) v.assign(2 * (size_t)nparts, 0);
+    auto first = [&](int t) { return (int)((long long)n * t / nt); };
+    host_chunks(nt, nt, [&](int b, int e) {
+        for (int t = b; t < e; ++t)
+            for (int r = first(t); r < first(t + 1); ++r) ++next[t][2 * part[r] + bnd[r]];
+    });
+    for (int p = 0; p < nparts; ++p)
     {
-        ++R.parts[part[r]].nloc;
-        R.parts[part[r]].nb += bnd[r];
+        ResPart& P = R.parts[p];
+        for (int t = 0; t < nt; ++t) P.nb += next[t][2 * p + 1];
+        int at[2] = {P.nb, 0};
+        for (int t = 0; t < nt; ++t)
+            for (int k = 0; k < 2; ++k)
+            {
+                const int c = next[t][2 * p + k];
+                next[t][2 * p + k] = at[k];
+                at[k] += c;
+            }
+        P.nloc = at[0];
     }
     R.maxLocP = 0;
     R.rowsP = 0;
@@ -286,16 +302,15 @@ bool res_partition(int n, const HostLayout& L, bool ordered, int nparts, ResHost
         R.maxLocP = std::max(R.maxLocP, p.nlocP);
     }
     R.rowMap.assign((size_t)R.rowsP, -1);
-    {
-        std::vector<int32_t> nextB(nparts, 0), nextI(nparts);
-        for (int p = 0; p < nparts; ++p) nextI[p] = R.parts[p].nb;
-        for (int r = 0; r < n; ++r)
-        {
-            const int p = part[r];
-            loc[r] = bnd[r] ? nextB[p]++ : nextI[p]++;
-            R.rowMap[(size_t)R.parts[p].rowBase + loc[r]] = r;
-        }
-    }
+    host_chunks(nt, nt, [&](int b, int e) {
+        for (int t = b; t < e; ++t)
+            for (int r = first(t); r < first(t + 1); ++r)
+            {
+                const int p = part[r];
+                loc[r] = next[t][2 * p + bnd[r]]++;
+                R.rowMap[(size_t)R.parts[p].rowBase + loc[r]] = r;
+            }
+    });
     R.idx.resize((size_t)R.rowsP * W);
     R.emap.assign((size_t)R.rowsP * W, -1);
     std::vector<std::vector<int32_t>> halo(nparts);

@@ -860,15 +860,11 @@ void resident_build(cf_context* c)
     const int nparts = std::min(c->numSMs, RES_MAX_PARTS);
     if (!c->coopLaunch || c->n > (long long)nparts * RES_MAX_ROWS || c->hostSliceOff.empty()) return;
     ResPlan* p = nullptr;
-    try
     {
-        if (res_plan_build(c->device, c->n, host_layout(c), !c->identityPerm, nparts, 0, 0,
-                           c->stream, &p) != CF_OK)
+        const LentLayout lent(c);
+        if (res_plan_build(c->device, c->n, lent.L, !c->identityPerm, nparts, 0, 0, c->stream,
+                           &p) != CF_OK)
             cudaGetLastError();   // no memory for the split: the graph path
-    }
-    catch (...)
-    {
-        return;                   // (for the host's copy of the layout)
     }
     if (p && p->maxHalo > SPLIT_MAX_HALO)
     {
